@@ -139,6 +139,7 @@ struct dtb_ctx {
     GainUnit* units = nullptr;
     int n_units = 0;
     int gain_grid = 0;
+    GainPass gain_pass;
     int f_smem_len = 0;
     int* unit_ptr = nullptr;
     double* partial = nullptr;

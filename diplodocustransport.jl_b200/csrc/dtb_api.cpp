@@ -667,14 +667,39 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
             g.host.shrink_to_fit();
         }
     }
+    // binary domain: `in(off_space, Domain)` per cell (entries outside 0..n_space-1 match no cell)
+    ops.bin_on = nullptr;
+    c->n_bin_cells = c->n_space;
+    c->bin_cells = nullptr;
+    if (c->has_bin_domain) {
+        std::vector<int> on((size_t)c->n_space, 0), list;
+        for (int64_t k : c->bin_domain)
+            if (k >= 0 && k < c->n_space) on[(size_t)k] = 1;
+        for (int k = 0; k < c->n_space; ++k)
+            if (on[(size_t)k]) list.push_back(k);
+        std::vector<unsigned char> on8(on.begin(), on.end());
+        unsigned char* d_on;
+        DTB_TRY(c->alloc(&d_on, on8.size()));
+        DTB_CUDA(cudaMemcpyAsync(d_on, on8.data(), on8.size(), cudaMemcpyHostToDevice, c->stream));
+        DTB_CUDA(cudaStreamSynchronize(c->stream));
+        ops.bin_on = d_on;
+        c->n_bin_cells = (int)list.size();
+        if (!list.empty()) DTB_TRY(copy_host_ints(c, &c->bin_cells, list));
+    }
     // work units, ordered by output row
     c->f_smem_len = (int)c->offp[c->ns];
-    int bps = gain_stream_blocks_per_sm((int)esz, c->f_smem_len);
+    int max_n2p = 8;
+    for (auto& b : blks) max_n2p = std::max(max_n2p, (int)b.n2p);
+    for (auto& sb : sblks)
+        for (auto& R : sb.runs) max_n2p = std::max(max_n2p, R.w);
+    c->gain_pass = gain_pass((int)esz, c->f_smem_len, max_n2p, std::max(1, c->n_bin_cells));
+    int bps = gain_stream_blocks_per_sm((int)esz, c->gain_pass, c->f_smem_len);
     DTB_CHECK(bps >= 1 || (blks.empty() && sblks.empty()), DTB_EINVAL,
               "gain kernel does not fit on an SM (state vector too long)");
     if (bps < 1) bps = 1;
     std::vector<GainUnit> units;
     std::vector<int> unit_ptr((size_t)c->n_mom + 1, 0);
+    int unit_row = 0;
     {
         double tot_bytes = sparse_bytes;
         for (auto& b : blks) tot_bytes += (double)b.no * b.n1 * b.n2 * esz;
@@ -683,49 +708,72 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
         std::vector<std::vector<std::pair<const SpBlk*, const SparseRun*>>> srow((size_t)c->n_mom);
         for (auto& sb : sblks)
             for (auto& R : sb.runs) srow[(size_t)(c->off[sb.out] + R.al)].push_back({&sb, &R});
-        // about 8 work units per CTA spread the HBM stream of a large G evenly; an L2-resident G
-        // (64 MB or less) is bound by the per-unit round trip of the tile ring instead, so its
-        // units are about 8 times larger (config 0: 14.8 against 15.6 us per step)
-        const double units_per_cta = tot_bytes <= 64.0 * 1024 * 1024 ? 1.0 : 8.0;
-        const double target = std::min(256.0 * 1024, std::max((double)kGainTileBytes,
-                                                               tot_bytes / ((double)c->num_sms * bps * units_per_cta)));
-        for (int64_t a = 0; a < c->n_mom; ++a) {
-            unit_ptr[(size_t)a] = (int)units.size();
-            const int sa = species_of(c, a);
-            for (auto& b : blks) {
-                if (b.out != sa) continue;
-                const int64_t al = a - c->off[sa];
-                const int64_t row_b = b.n2p * (int64_t)esz;
-                const int tile_b = (int)std::max<int64_t>(1, std::min<int64_t>(b.n1, kGainTileBytes / row_b));
-                int64_t nb = std::max<int64_t>(tile_b, (int64_t)(target / row_b) / tile_b * tile_b);
-                for (int64_t b0 = 0; b0 < b.n1; b0 += nb) {
+        // The units in row order, dense blocks in pieces of about `target` bytes (whole tiles).
+        const auto each_unit = [&](double target, auto&& emit) {
+            for (int64_t a = 0; a < c->n_mom; ++a) {
+                const int sa = species_of(c, a);
+                for (auto& b : blks) {
+                    if (b.out != sa) continue;
+                    const int64_t al = a - c->off[sa];
+                    const int64_t row_b = b.n2p * (int64_t)esz;
+                    const int tile_b = (int)std::max<int64_t>(1, std::min<int64_t>(b.n1, kGainTileBytes / row_b));
+                    const int64_t nb = std::max<int64_t>(tile_b, (int64_t)(target / row_b) / tile_b * tile_b);
+                    for (int64_t b0 = 0; b0 < b.n1; b0 += nb) {
+                        GainUnit u;
+                        u.g_off = b.elem_off + (al * b.n1 + b0) * b.n2p;
+                        u.b_off = (int)(c->offp[b.in1] + b0);
+                        u.c_off = (int)c->offp[b.in2];
+                        u.nb = (int)std::min(nb, b.n1 - b0);
+                        u.n2p = (int)b.n2p;
+                        u.tile_b = tile_b;
+                        u.row = (int)a;
+                        emit(u);
+                    }
+                }
+                for (auto& pr : srow[(size_t)a]) {
+                    const SpBlk& sb = *pr.first;
+                    const SparseRun& R = *pr.second;
+                    const int tile_b =
+                        (int)std::max<int64_t>(1, std::min<int64_t>(R.nb, kGainTileBytes / (R.w * (int64_t)esz)));
                     GainUnit u;
-                    u.g_off = b.elem_off + (al * b.n1 + b0) * b.n2p;
-                    u.b_off = (int)(c->offp[b.in1] + b0);
-                    u.c_off = (int)c->offp[b.in2];
-                    u.nb = (int)std::min(nb, b.n1 - b0);
-                    u.n2p = (int)b.n2p;
+                    u.g_off = sb.elem_off + R.elem_off;
+                    u.b_off = (int)(c->offp[sb.in1] + R.b0);
+                    u.c_off = (int)(c->offp[sb.in2] + R.c0);
+                    u.nb = R.nb;
+                    u.n2p = R.w;
                     u.tile_b = tile_b;
                     u.row = (int)a;
-                    units.push_back(u);
+                    emit(u);
                 }
             }
-            for (auto& pr : srow[(size_t)a]) {
-                const SpBlk& sb = *pr.first;
-                const SparseRun& R = *pr.second;
-                const int tile_b = (int)std::max<int64_t>(1, std::min<int64_t>(R.nb, kGainTileBytes / (R.w * (int64_t)esz)));
-                GainUnit u;
-                u.g_off = sb.elem_off + R.elem_off;
-                u.b_off = (int)(c->offp[sb.in1] + R.b0);
-                u.c_off = (int)(c->offp[sb.in2] + R.c0);
-                u.nb = R.nb;
-                u.n2p = R.w;
-                u.tile_b = tile_b;
-                u.row = (int)a;
-                units.push_back(u);
+        };
+        // The CTAs take the units round robin, so a size is judged by the fullest CTA: its bytes
+        // plus, per unit, about what a unit's reduction costs in streaming time. At most about 32
+        // units per CTA are looked at. (Against eight units per CTA whatever the remainder: 44.3
+        // against 46.4 us per step on one cell of 2 x 256 FP64 states, 61 against 71 on eight.)
+        const size_t ctas = (size_t)c->num_sms * bps;
+        const double unit_cost = 4096.0 + 1024.0 * c->gain_pass.cells;
+        double target = kGainTileBytes, best = 0;
+        std::vector<double> load(ctas);
+        for (double t = 256.0 * 1024; t >= kGainTileBytes; t -= t > 128.0 * 1024 ? 32768 : 16384) {
+            if (t * 32.0 * (double)ctas < tot_bytes && best > 0) break;
+            std::fill(load.begin(), load.end(), 0.0);
+            size_t k = 0;
+            each_unit(t, [&](const GainUnit& u) {
+                load[k] += (double)u.nb * u.n2p * esz + unit_cost;
+                if (++k == ctas) k = 0;
+            });
+            const double m = *std::max_element(load.begin(), load.end());
+            if (best == 0 || m < best) {
+                best = m;
+                target = t;
             }
         }
-        unit_ptr[(size_t)c->n_mom] = (int)units.size();
+        each_unit(target, [&](const GainUnit& u) {
+            while (unit_row < u.row) unit_ptr[(size_t)++unit_row] = (int)units.size();
+            units.push_back(u);
+        });
+        while (unit_row < c->n_mom) unit_ptr[(size_t)++unit_row] = (int)units.size();
     }
     c->n_units = (int)units.size();
     c->gain_grid = std::max(1, std::min(c->n_units, c->num_sms * bps));
@@ -868,25 +916,6 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
     ops.n_units = c->n_units;
     ops.partial = c->partial;
     ops.thr = c->prec == DTB_F64 ? (double)1e-10f : (double)(T)1e-10f;
-    // binary domain: `in(off_space, Domain)` per cell (entries outside 0..n_space-1 match no cell)
-    ops.bin_on = nullptr;
-    c->n_bin_cells = c->n_space;
-    c->bin_cells = nullptr;
-    if (c->has_bin_domain) {
-        std::vector<int> on((size_t)c->n_space, 0), list;
-        for (int64_t k : c->bin_domain)
-            if (k >= 0 && k < c->n_space) on[(size_t)k] = 1;
-        for (int k = 0; k < c->n_space; ++k)
-            if (on[(size_t)k]) list.push_back(k);
-        std::vector<unsigned char> on8(on.begin(), on.end());
-        unsigned char* d_on;
-        DTB_TRY(c->alloc(&d_on, on8.size()));
-        DTB_CUDA(cudaMemcpyAsync(d_on, on8.data(), on8.size(), cudaMemcpyHostToDevice, c->stream));
-        DTB_CUDA(cudaStreamSynchronize(c->stream));
-        ops.bin_on = d_on;
-        c->n_bin_cells = (int)list.size();
-        if (!list.empty()) DTB_TRY(copy_host_ints(c, &c->bin_cells, list));
-    }
     ops.has_bin = c->has_bin;
     ops.has_emi = c->has_emi;
     return DTB_OK;
@@ -984,7 +1013,7 @@ static int launch_step(dtb_ctx* c, RowOps<T>& ops, double dt_imm, bool use_arr, 
             e1 = c->ev[k + 1];
             DTB_CUDA(cudaEventRecord(e0, c->stream));
         }
-        DTB_CUDA(launch_gain_stream<T>(reinterpret_cast<const T*>(c->G_all), c->units, c->n_units, fin, (int)c->n_mom,
+        DTB_CUDA(launch_gain_stream<T>(c->gain_pass, reinterpret_cast<const T*>(c->G_all), c->units, c->n_units, fin, (int)c->n_mom,
                                        c->sp_off_host, c->ns, c->f_smem_len, c->partial, c->n_bin_cells,
                                        c->gain_grid, c->err, c->stream, c->bin_cells, true));
         c->launches++;

@@ -94,10 +94,20 @@ struct RowOps {
 };
 
 // Launch helpers (kernels_plain.cu).
+
+// Shape of a gain pass: space cells that share one read of G, and 16-byte G columns per thread.
+struct GainPass {
+    int cells = 1;
+    int kv = 1;
+};
+constexpr int kGainMaxCells = 8;
+constexpr int kGainSmemLimit = 232448;  // shared memory a CTA may have on sm_100
+GainPass gain_pass(int elem_size, int f_smem_len, int max_n2p, int n_cells);
+
 template <typename T>
-cudaError_t launch_gain_stream(const T* G, const GainUnit* units, int n_units, const T* f,
-                               int n_mom, const int* sp_offp_dev, int n_species, int f_smem_len,
-                               double* partial, int n_space, int grid_x, int* err, cudaStream_t s,
+cudaError_t launch_gain_stream(const GainPass& pass, const T* G, const GainUnit* units, int n_units, const T* f,
+                               int n_mom, const int* sp_off_host, int n_species, int f_smem_len,
+                               double* partial, int n_cells, int grid_x, int* err, cudaStream_t s,
                                const int* cell_list = nullptr, bool pdl = false);
 
 // Fields of one row block's diagnostics record: min cr, cr_bin, cr_emi, cr_flux, sum df, sum f.
@@ -139,8 +149,8 @@ cudaError_t launch_moments_f32(const float* f, int n_mom, int n_space, const int
 
 cudaError_t launch_bounded_wait_selftest(unsigned long long limit_ns, int* err, cudaStream_t s);
 
-int gain_stream_smem_bytes(int elem_size, int f_smem_len);
-int gain_stream_blocks_per_sm(int elem_size, int f_smem_len);
+int gain_stream_smem_bytes(int elem_size, int f_smem_len, int cells);
+int gain_stream_blocks_per_sm(int elem_size, const GainPass& pass, int f_smem_len);
 constexpr int kGainTileBytes = 16384;
 constexpr int kGainStages = 4;
 constexpr int kGainConsumerWarps = 8;

@@ -145,7 +145,8 @@ int gain_op_run(int32_t dtype, const void* G, int64_t n_out, int64_t n1, int64_t
     int sp[6] = {0, (int)n1, (int)(n1 + n2), 0, (int)offp1, (int)(offp1 + n2)};
     const int f_len = (int)(offp1 + n2);
     const int n_state = (int)(n1 + n2);
-    const int bps = gain_stream_blocks_per_sm(esz, f_len);
+    const GainPass pass = gain_pass(esz, f_len, (int)n2, 1);
+    const int bps = gain_stream_blocks_per_sm(esz, pass, f_len);
     if (bps < 1) {
         set_error("gain op: vectors too long for the shared-memory stage");
         return DTB_EINVAL;
@@ -155,10 +156,10 @@ int gain_op_run(int32_t dtype, const void* G, int64_t n_out, int64_t n1, int64_t
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = std::max(1, std::min(n_units, sms * bps));
     if (dtype == DTB_DTYPE_F64)
-        e = launch_gain_stream<double>(static_cast<const double*>(G), d_units, n_units,
+        e = launch_gain_stream<double>(pass, static_cast<const double*>(G), d_units, n_units,
                                        reinterpret_cast<const double*>(d_f), n_state, sp, 2, f_len, d_part, 1, grid, err, s);
     else
-        e = launch_gain_stream<float>(static_cast<const float*>(G), d_units, n_units,
+        e = launch_gain_stream<float>(pass, static_cast<const float*>(G), d_units, n_units,
                                       reinterpret_cast<const float*>(d_f), n_state, sp, 2, f_len, d_part, 1, grid, err, s);
     if (e == cudaSuccess) e = launch_row_sums(d_part, (int)n_out, plan.splits, out, s);
     if (e != cudaSuccess) {
@@ -209,7 +210,9 @@ extern "C" int32_t dtb_gain_contract(int32_t dtype, const void* G, int64_t n_out
     }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     GainOpPlan plan;
-    rc = gain_op_plan(n_out, n1, n2, esz, sms, gain_stream_blocks_per_sm(esz, (int)((n1 + 7) / 8 * 8 + n2)), plan);
+    const int f_len = (int)((n1 + 7) / 8 * 8 + n2);
+    rc = gain_op_plan(n_out, n1, n2, esz, sms, gain_stream_blocks_per_sm(esz, gain_pass(esz, f_len, (int)n2, 1), f_len),
+                      plan);
     if (rc != DTB_OK) return rc;
     const size_t need = gain_op_scratch_bytes(plan.n_units, n1, n2, esz);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);

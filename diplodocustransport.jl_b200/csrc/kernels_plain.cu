@@ -2,8 +2,9 @@
 //
 // One step is two launches,
 //   gain_stream  - streams the gain blocks G[a][b][c] from HBM through a bulk-copy (TMA)
-//                  pipeline in shared memory and contracts each tile against f_b f_c formed
-//                  on the fly; writes one FP64 partial per (row, b-range) work unit.
+//                  pipeline in shared memory and contracts each tile against f_b, then each
+//                  work unit (a row and a range of b) against f_c, for up to eight space cells
+//                  per read of G; writes one FP64 partial per unit and cell.
 //   euler_rows   - one warp per state row: banded flux row (ELL, 128-bit loads), emission
 //                  row pieces, loss bilinear term, sum of the row's gain partials, then the
 //                  Euler update and clamp of SteppingMethods.jl:46-101; each block writes a
@@ -15,6 +16,8 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "dtb_internal.h"
 #include "pdl.cuh"
@@ -95,63 +98,204 @@ struct SpOff {
     int offp[DTB_MAX_SPECIES + 1];  // padded (multiples of 8)
 };
 
+// 16 bytes of G as FP64 values.
 template <typename T>
 struct Vec;
 template <>
 struct Vec<float> {
     using type = float4;
     static constexpr int n = 4;
-    __device__ __forceinline__ static float dot(const float4& a, const float4& b) {
-        return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
+    __device__ __forceinline__ static void unpack(const float4& g, double (&v)[4]) {
+        v[0] = g.x;
+        v[1] = g.y;
+        v[2] = g.z;
+        v[3] = g.w;
     }
 };
 template <>
 struct Vec<double> {
     using type = double2;
     static constexpr int n = 2;
-    __device__ __forceinline__ static double dot(const double2& a, const double2& b) {
-        return a.x * b.x + a.y * b.y;
+    __device__ __forceinline__ static void unpack(const double2& g, double (&v)[2]) {
+        v[0] = g.x;
+        v[1] = g.y;
     }
 };
 
 constexpr int kGainThreads = (kGainConsumerWarps + 1) * 32;
+constexpr int kGainConsumers = kGainConsumerWarps * 32;
 
 __host__ __device__ constexpr int round_up_int(int x, int m) { return (x + m - 1) / m * m; }
+__host__ __device__ constexpr int pow2_ceil(int x) { return x <= 1 ? 1 : 2 * pow2_ceil((x + 1) / 2); }
 
 // Reduction ring: a consumer warp can run at most kGainStages tiles (hence units) ahead of
 // warp 0, so kGainStages + 2 slots never alias a slot warp 0 is still reading.
 constexpr int kRedRing = kGainStages + 2;
 
-int gain_stream_smem_bytes(int elem_size, int f_smem_len) {
-    return kGainStages * kGainTileBytes + round_up_int(f_smem_len * elem_size, 16) + 2 * kGainStages * 8 +
-           kRedRing * 8 + kRedRing * kGainConsumerWarps * 8 + 16;
+// Staged states: in the state type for one cell, FP64 for several (one conversion per state and
+// block, not one per b-row).
+template <typename T, int C>
+struct StagedT {
+    using type = double;
+};
+template <typename T>
+struct StagedT<T, 1> {
+    using type = T;
+};
+
+int gain_stream_smem_bytes(int elem_size, int f_smem_len, int cells) {
+    return kGainStages * kGainTileBytes + round_up_int(f_smem_len * cells * (cells == 1 ? elem_size : 8), 16) +
+           2 * kGainStages * 8 + kRedRing * 8 + kRedRing * (int)sizeof(GainUnit) +
+           kRedRing * kGainConsumerWarps * cells * 8 + 16;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kGainThreads) gain_stream_kernel(const T* __restrict__ G,
+// Sums of N values over the warp's 32 lanes: halving exchanges while several values are left,
+// then a butterfly. Lane l of the result holds value l >> (5 - log2 N). Every value is summed by
+// the same tree (lane distances 16, 8, 4, 2, 1), so its bits do not depend on N.
+template <int N>
+__device__ __forceinline__ double warp_sum_n(double (&v)[N], int lane) {
+    int o = 16;
+#pragma unroll
+    for (int n = N; n > 1; n /= 2, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            if (i < n / 2) {
+                const double send = up ? v[i] : v[i + n / 2];
+                const double keep = up ? v[i + n / 2] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+    }
+#pragma unroll
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
+// Thread `tid`'s share of one work unit: the 16-byte columns cv, cv + w, .. (KV of them, w threads
+// to a b-row) of b-rows r0, r0 + dr, .. of every tile.
+struct UnitMap {
+    int nvr, w, dr, r0, cv;
+    bool on;
+};
+template <typename T, int KV>
+__device__ __forceinline__ UnitMap unit_map(const GainUnit& U, int tid) {
+    UnitMap m;
+    m.nvr = U.n2p / Vec<T>::n;
+    m.w = (m.nvr + KV - 1) / KV;
+    m.dr = kGainConsumers / m.w;
+    m.r0 = tid / m.w;
+    m.cv = tid - m.r0 * m.w;
+    m.on = m.r0 < m.dr;
+    return m;
+}
+
+// y[kv][c][e] += f1[b][c] G[b][column kv, element e] over the thread's b-rows of one tile, in
+// order. FP64 throughout: with one cell that is 2 (FP64) or 4 (FP32) FMAs per 16 bytes, and one
+// broadcast read of f1 per row; with C cells the tile is read once for all of them.
+template <typename T, int C, int KV>
+__device__ __forceinline__ void tile_accumulate(const UnitMap& m, const unsigned char* tile, int rows,
+                                                const typename StagedT<T, C>::type* f1, int f_len,
+                                                double (&y)[KV][C][Vec<T>::n]) {
+    using V = Vec<T>;
+    using vec_t = typename V::type;
+    if (!m.on) return;
+    const vec_t* tv = reinterpret_cast<const vec_t*>(tile);
+    constexpr int kUnroll = KV * C * V::n <= 8 ? 2 : 1;
+#pragma unroll kUnroll
+    for (int r = m.r0; r < rows; r += m.dr) {
+        double g[KV][V::n];
+#pragma unroll
+        for (int k = 0; k < KV; ++k) {
+            // a column past the row's end repeats the last one; its sum is not used
+            const int cv = k == 0 ? m.cv : min(m.cv + k * m.w, m.nvr - 1);
+            V::unpack(tv[r * m.nvr + cv], g[k]);
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const double x = (double)f1[c * f_len + r];
+#pragma unroll
+            for (int k = 0; k < KV; ++k)
+#pragma unroll
+                for (int e = 0; e < V::n; ++e) y[k][c][e] = fma(x, g[k][e], y[k][c][e]);
+        }
+    }
+}
+
+// The unit's contraction with f2 and the warp's sum; lane l holds cell l >> (5 - log2 pow2_ceil(C)).
+template <typename T, int C, int KV>
+__device__ __forceinline__ double unit_warp_sum(const UnitMap& m, const typename StagedT<T, C>::type* f2, int f_len,
+                                                double (&y)[KV][C][Vec<T>::n], int lane) {
+    using V = Vec<T>;
+    double acc[pow2_ceil(C)];
+#pragma unroll
+    for (int c = 0; c < pow2_ceil(C); ++c) acc[c] = 0.0;
+    if (m.on) {
+#pragma unroll
+        for (int k = 0; k < KV; ++k) {
+            if (k == 0 || m.cv + k * m.w < m.nvr) {
+                const typename StagedT<T, C>::type* x = f2 + (m.cv + k * m.w) * V::n;
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+#pragma unroll
+                    for (int e = 0; e < V::n; ++e) acc[c] = fma((double)x[c * f_len + e], y[k][c][e], acc[c]);
+            }
+        }
+    }
+    return warp_sum_n<pow2_ceil(C)>(acc, lane);
+}
+
+// The cells of a pass, padded per species ([cell][state]: the lanes of a warp read consecutive
+// states of one cell); zeros in the padding and for cells past the last.
+template <typename T, int C>
+__device__ __forceinline__ void stage_f(typename StagedT<T, C>::type* f_s, const T* __restrict__ f, const SpOff& so,
+                                        int f_len, int n_mom, const int* cell_list, int cell0, int n_cells, int tid,
+                                        int n_threads) {
+    for (int i = tid; i < f_len; i += n_threads) {
+        int s = 0;
+        while (s + 1 < so.n && i >= so.offp[s + 1]) ++s;
+        const int j = i - so.offp[s];
+        const bool in = j < so.off[s + 1] - so.off[s];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            T v = T(0);
+            if (in && cell0 + c < n_cells) {
+                const int cell = cell_list ? cell_list[cell0 + c] : cell0 + c;
+                v = f[(size_t)cell * n_mom + so.off[s] + j];
+            }
+            f_s[c * f_len + i] = v;
+        }
+    }
+}
+
+// One block streams work units through a ring of 16 KB tiles for up to C space cells at once
+// (grid y: groups of C cells), so G crosses HBM once per group and not once per cell. Bound: HBM
+// with one cell (2 x 1024 states in FP32: 6.5 TB/s, the copy rate); with eight FP64 cells the
+// shared-memory reads and the work per 16 KB tile (4.8 TB/s of G on 2 x 256 states). At most 96
+// registers: two CTAs of nine warps per SM.
+template <typename T, int C, int KV>
+__global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* __restrict__ G,
                                                                    const GainUnit* __restrict__ units,
                                                                    int n_units, const T* __restrict__ f,
                                                                    int n_mom, SpOff so, int f_len,
                                                                    double* __restrict__ partial, int* err,
-                                                                   const int* __restrict__ cell_list) {
-    using V = Vec<T>;
-    using vec_t = typename V::type;
+                                                                   const int* __restrict__ cell_list, int n_cells) {
     constexpr int kTileElems = kGainTileBytes / sizeof(T);
-    constexpr int kNC = kGainConsumerWarps * 32;
+    constexpr int kMaxVec = KV * kGainConsumers;
 
     extern __shared__ __align__(128) unsigned char smem[];
-    T* stage_base = reinterpret_cast<T*>(smem);
-    T* f_s = reinterpret_cast<T*>(smem + kGainStages * kGainTileBytes);
+    using S = typename StagedT<T, C>::type;
+    S* f_s = reinterpret_cast<S*>(smem + kGainStages * kGainTileBytes);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kGainStages * kGainTileBytes +
-                                                 round_up_int(f_len * (int)sizeof(T), 16));
+                                                 round_up_int(f_len * C * (int)sizeof(S), 16));
     uint64_t* empty = full + kGainStages;
     uint64_t* unit_bar = empty + kGainStages;
-    double* red = reinterpret_cast<double*>(unit_bar + kRedRing);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(red + kRedRing * kGainConsumerWarps);
+    GainUnit* unit_s = reinterpret_cast<GainUnit*>(unit_bar + kRedRing);  // the work records, by unit slot
+    double* red = reinterpret_cast<double*>(unit_s + kRedRing);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(red + kRedRing * kGainConsumerWarps * C);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // the cells of the binary domain, or every cell when there is no list
-    const int cell = cell_list ? cell_list[blockIdx.y] : (int)blockIdx.y;
+    const int cell0 = blockIdx.y * C;
 
     if (tid == 0) {
         for (int s = 0; s < kGainStages; ++s) {
@@ -164,15 +308,21 @@ __global__ void __launch_bounds__(kGainThreads) gain_stream_kernel(const T* __re
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();  // barriers initialised; the producer may stream G before f is ready
+    const auto bad = [](const GainUnit& U) {
+        return U.nb <= 0 || U.tile_b <= 0 || U.n2p <= 0 || U.tile_b * U.n2p > kTileElems || U.n2p / Vec<T>::n > kMaxVec;
+    };
 
     if (warp == kGainConsumerWarps) {
         // ---------------- producer: one thread issues the bulk copies
         if (lane == 0) {
-            uint32_t it = 0;
+            uint32_t it = 0, lk = 0;
             bool ok = true;
-            for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-                const GainUnit U = units[u];
-                if (U.tile_b <= 0 || U.n2p <= 0 || U.tile_b * U.n2p > kTileElems) {
+            GainUnit N{};
+            if ((int)blockIdx.x < n_units) N = units[blockIdx.x];
+            for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++lk) {
+                const GainUnit U = N;
+                if (u + (int)gridDim.x < n_units) N = units[u + gridDim.x];  // in flight beside this unit
+                if (bad(U)) {
                     atomicOr(err, KERR_BAD_UNIT);
                     *abort_flag = 1;
                     ok = false;
@@ -188,11 +338,14 @@ __global__ void __launch_bounds__(kGainThreads) gain_stream_kernel(const T* __re
                         ok = false;
                         break;
                     }
+                    // the record reaches the consumers with the unit's first tile; its slot is free:
+                    // a unit kRedRing back was reduced before this stage was released
+                    if (t == 0) unit_s[lk % kRedRing] = U;
                     const int rows = min(U.tile_b, U.nb - t * U.tile_b);
                     const uint32_t bytes = (uint32_t)rows * (uint32_t)U.n2p * (uint32_t)sizeof(T);
                     mbar_arrive_expect_tx(smem_u32(&full[st]), bytes);
-                    bulk_g2s(smem_u32(stage_base + (size_t)st * kTileElems),
-                             G + U.g_off + (long long)t * U.tile_b * U.n2p, bytes, smem_u32(&full[st]));
+                    bulk_g2s(smem_u32(smem + (size_t)st * kGainTileBytes), G + U.g_off + (long long)t * U.tile_b * U.n2p,
+                             bytes, smem_u32(&full[st]));
                 }
             }
             // Wait for this block's own copies before the block may exit.
@@ -207,36 +360,22 @@ __global__ void __launch_bounds__(kGainThreads) gain_stream_kernel(const T* __re
     }
 
     // ---------------- consumers: 8 warps
-    // The work table is static: the block's first unit is read before the wait.
-    GainUnit U0{};
-    if ((int)blockIdx.x < n_units) U0 = units[blockIdx.x];
     // f is the previous step's output and the previous step still reads the partials this
     // kernel writes: wait for it (the G tiles already stream in meanwhile)
     pdl_wait();
     if (tid == 0) pdl_trigger();
-    {
-        // f of this cell in the padded per-species layout; zeros in the padding.
-        const T* fc = f + (size_t)cell * n_mom;
-        for (int i = tid; i < f_len; i += kNC) {
-            int s = 0;
-            while (s + 1 < so.n && i >= so.offp[s + 1]) ++s;
-            const int j = i - so.offp[s];
-            const int ns = so.off[s + 1] - so.off[s];
-            f_s[i] = (j < ns) ? fc[so.off[s] + j] : T(0);
-        }
-    }
-    asm volatile("bar.sync 1, %0;" ::"n"(kNC) : "memory");  // the consumer warps only
+    stage_f<T, C>(f_s, f, so, f_len, n_mom, cell_list, cell0, n_cells, tid, kGainConsumers);
+    asm volatile("bar.sync 1, %0;" ::"n"(kGainConsumers) : "memory");  // the consumer warps only
     uint32_t it = 0;
     uint32_t lk = 0;  // units done by this block
     for (int u = blockIdx.x; u < n_units; u += gridDim.x, ++lk) {
-        const GainUnit U = u == (int)blockIdx.x ? U0 : units[u];
-        if (U.tile_b <= 0 || U.n2p <= 0 || U.tile_b * U.n2p > kTileElems) return;
-        const int nt = (U.nb + U.tile_b - 1) / U.tile_b;
-        const int nvr = U.n2p / V::n;  // vectors per b-row
-        const int dr = kNC / nvr, dcv = kNC - dr * nvr;
-        const T* f2 = f_s + U.c_off;
-        double acc = 0.0;
-        for (int t = 0; t < nt; ++t, ++it) {
+        const int slot = lk % kRedRing;
+        const GainUnit* U = &unit_s[slot];  // valid from the unit's first tile on
+        UnitMap m{};
+        double y[KV][C][Vec<T>::n] = {};
+        const S* f1 = f_s;
+        int left = 1, tile_b = 0;  // b-rows left; at least one tile
+        for (; left > 0; left -= tile_b, f1 += tile_b, ++it) {
             const int st = it % kGainStages;
             const uint32_t ph = (it / kGainStages) & 1u;
             if (!mbar_wait_bounded(smem_u32(&full[st]), ph, abort_flag)) {
@@ -244,64 +383,104 @@ __global__ void __launch_bounds__(kGainThreads) gain_stream_kernel(const T* __re
                 *abort_flag = 1;
                 return;
             }
-            const int rows = min(U.tile_b, U.nb - t * U.tile_b);
-            const vec_t* tile = reinterpret_cast<const vec_t*>(stage_base + (size_t)st * kTileElems);
-            const T* f1 = f_s + U.b_off + t * U.tile_b;
-            int r = tid / nvr, cv = tid - r * nvr;
-            while (r < rows) {
-                const vec_t g = tile[r * nvr + cv];
-                const vec_t x = reinterpret_cast<const vec_t*>(f2)[cv];
-                const T d = V::dot(g, x);
-                acc = fma((double)f1[r], (double)d, acc);
-                cv += dcv;
-                r += dr;
-                if (cv >= nvr) {
-                    cv -= nvr;
-                    ++r;
-                }
+            if (tile_b == 0) {
+                m = unit_map<T, KV>(*U, tid);
+                f1 += U->b_off;
+                left = U->nb;
+                tile_b = U->tile_b;
             }
+            tile_accumulate<T, C, KV>(m, smem + (size_t)st * kGainTileBytes, min(tile_b, left), f1, f_len, y);
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&empty[st]));
         }
-        acc = warp_sum(acc);
-        const int slot = lk % kRedRing;
-        if (lane == 0) {
-            red[slot * kGainConsumerWarps + warp] = acc;
-            mbar_arrive(smem_u32(&unit_bar[slot]));
-        }
-        if (tid == 0) {
+        const double acc = unit_warp_sum<T, C, KV>(m, f_s + U->c_off, f_len, y, lane);
+        constexpr int kLanes = 32 / pow2_ceil(C);  // lanes per cell of the warp's sums
+        if (lane % kLanes == 0 && lane / kLanes < C) red[(slot * kGainConsumerWarps + warp) * C + lane / kLanes] = acc;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&unit_bar[slot]));
+        if (warp == 0) {
             if (!mbar_wait_bounded(smem_u32(&unit_bar[slot]), (lk / kRedRing) & 1u, abort_flag)) {
                 if (!*abort_flag) atomicOr(err, KERR_TIMEOUT_FULL);
                 *abort_flag = 1;
                 return;
             }
-            double s = 0.0;
+            if (lane < C && cell0 + lane < n_cells) {
+                double s = 0.0;
 #pragma unroll
-            for (int w = 0; w < kGainConsumerWarps; ++w) s += red[slot * kGainConsumerWarps + w];
-            partial[(size_t)cell * n_units + u] = s;
+                for (int w = 0; w < kGainConsumerWarps; ++w) s += red[(slot * kGainConsumerWarps + w) * C + lane];
+                const int cell = cell_list ? cell_list[cell0 + lane] : cell0 + lane;
+                partial[(size_t)cell * n_units + u] = s;
+            }
         }
     }
 }
 
-int gain_stream_blocks_per_sm(int elem_size, int f_smem_len) {
+namespace {
+
+template <typename T>
+using GainKernel = void (*)(const T*, const GainUnit*, int, const T*, int, SpOff, int, double*, int*, const int*, int);
+
+// The instance of a pass (gain_pass picks only these): at most 32 FP64 accumulators per thread.
+template <typename T, int KV, int C>
+GainKernel<T> gain_kernel_upto(int cells) {
+    if constexpr (C > 1) {
+        if (cells < C) return gain_kernel_upto<T, KV, C - 1>(cells);
+    }
+    return gain_stream_kernel<T, C, KV>;
+}
+template <typename T>
+GainKernel<T> gain_kernel(const GainPass& p) {
+    constexpr int n = Vec<T>::n;
+    if (p.kv == 1) return gain_kernel_upto<T, 1, sizeof(T) == 8 ? 2 : 8>(p.cells);
+    if (p.kv == 2) return gain_kernel_upto<T, 2, 32 / (2 * n)>(p.cells);
+    return gain_kernel_upto<T, 4, 32 / (4 * n)>(p.cells);
+}
+
+template <typename T>
+int pass_blocks_per_sm(const GainPass& p, int f_smem_len) {
     int n = 0;
-    const int smem = gain_stream_smem_bytes(elem_size, f_smem_len);
-    if (elem_size == 8) {
-        cudaFuncSetAttribute(gain_stream_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gain_stream_kernel<double>, kGainThreads, smem);
-    } else {
-        cudaFuncSetAttribute(gain_stream_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gain_stream_kernel<float>, kGainThreads, smem);
+    const int smem = gain_stream_smem_bytes(sizeof(T), f_smem_len, p.cells);
+    const auto k = gain_kernel<T>(p);
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kGainThreads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
     return n;
 }
 
+}  // namespace
+
+// Cells that share one read of G: as many as fit a thread's accumulators (32 FP64 values, 8 cells
+// at most) and the staged states a CTA's shared memory, split evenly over the passes they take
+// (the least padding). G is the traffic: eight cells of a 2 x 256-state FP64 grid (268 MB of G)
+// take 61 us per step in one pass and 321 us in eight.
+// 16-byte columns per thread: as many as cover the longest b-row with 256 threads. With three or
+// more FP64 cells at least two, since every cell costs a broadcast read of f1 per b-row and two
+// columns share it (one FP64 FMA pair per read is too little to hide it behind).
+GainPass gain_pass(int elem_size, int f_smem_len, int max_n2p, int n_cells) {
+    GainPass p;
+    const int nvr = max_n2p * elem_size / 16;
+    p.kv = nvr <= kGainConsumers ? 1 : (nvr <= 2 * kGainConsumers ? 2 : 4);
+    if (elem_size == 8 && n_cells > 2) p.kv = std::max(p.kv, 2);
+    int most = std::min(kGainMaxCells, 32 / (p.kv * (16 / elem_size)));
+    while (most > 1 && gain_stream_smem_bytes(elem_size, f_smem_len, most) > kGainSmemLimit) --most;
+    if (elem_size == 8 && p.kv == 1) most = std::min(most, 2);
+    const int passes = (n_cells + most - 1) / most;
+    p.cells = passes > 0 ? (n_cells + passes - 1) / passes : 1;
+    return p;
+}
+
+int gain_stream_blocks_per_sm(int elem_size, const GainPass& p, int f_smem_len) {
+    return elem_size == 8 ? pass_blocks_per_sm<double>(p, f_smem_len) : pass_blocks_per_sm<float>(p, f_smem_len);
+}
+
 template <typename T>
-cudaError_t launch_gain_stream(const T* G, const GainUnit* units, int n_units, const T* f, int n_mom,
-                               const int* sp_off_host, int n_species, int f_smem_len, double* partial,
-                               int n_space, int grid_x, int* err, cudaStream_t s, const int* cell_list, bool pdl) {
-    // n_space: cells to run (grid y); cell_list maps them to cells, or null for 0..n_space-1
-    // sp_off_host: [0..n_species] unpadded then [0..n_species] padded offsets (host array)
+cudaError_t launch_gain_stream(const GainPass& pass, const T* G, const GainUnit* units, int n_units, const T* f,
+                               int n_mom, const int* sp_off_host, int n_species, int f_smem_len, double* partial,
+                               int n_cells, int grid_x, int* err, cudaStream_t s, const int* cell_list, bool pdl) {
+    // n_cells: cells to run (grid y: groups of pass.cells); cell_list maps them to cells, or null
+    // for 0..n_cells-1. sp_off_host: [0..n_species] unpadded then [0..n_species] padded offsets
     SpOff so;
     so.n = n_species;
     for (int i = 0; i <= n_species; ++i) {
@@ -309,24 +488,24 @@ cudaError_t launch_gain_stream(const T* G, const GainUnit* units, int n_units, c
         so.offp[i] = sp_off_host[n_species + 1 + i];
     }
     // the dynamic shared-memory limit was raised by gain_stream_blocks_per_sm at commit
-    const int smem = gain_stream_smem_bytes(sizeof(T), f_smem_len);
-    dim3 grid(grid_x, n_space);
+    const int smem = gain_stream_smem_bytes(sizeof(T), f_smem_len, pass.cells);
+    const auto k = gain_kernel<T>(pass);
+    dim3 grid(grid_x, (n_cells + pass.cells - 1) / pass.cells);
     // pdl: a step's own sequence (its G is static); a caller's G may be its predecessor's output,
     // which the producer (it starts before the dependency wait) must not read early
     if (pdl)
-        return launch_pdl(gain_stream_kernel<T>, grid, dim3(kGainThreads), (size_t)smem, s, G, units, n_units, f, n_mom,
-                          so, f_smem_len, partial, err, cell_list);
-    gain_stream_kernel<T><<<grid, kGainThreads, smem, s>>>(G, units, n_units, f, n_mom, so, f_smem_len, partial, err,
-                                                           cell_list);
+        return launch_pdl(k, grid, dim3(kGainThreads), (size_t)smem, s, G, units, n_units, f, n_mom, so, f_smem_len,
+                          partial, err, cell_list, n_cells);
+    k<<<grid, kGainThreads, smem, s>>>(G, units, n_units, f, n_mom, so, f_smem_len, partial, err, cell_list, n_cells);
     return cudaGetLastError();
 }
 
-template cudaError_t launch_gain_stream<double>(const double*, const GainUnit*, int, const double*, int,
-                                                const int*, int, int, double*, int, int, int*, cudaStream_t,
+template cudaError_t launch_gain_stream<double>(const GainPass&, const double*, const GainUnit*, int, const double*,
+                                                int, const int*, int, int, double*, int, int, int*, cudaStream_t,
                                                 const int*, bool);
-template cudaError_t launch_gain_stream<float>(const float*, const GainUnit*, int, const float*, int,
-                                               const int*, int, int, double*, int, int, int*, cudaStream_t,
-                                               const int*, bool);
+template cudaError_t launch_gain_stream<float>(const GainPass&, const float*, const GainUnit*, int, const float*, int,
+                                               const int*, int, int, double*, int, int, int*, cudaStream_t, const int*,
+                                               bool);
 
 // ------------------------------------------------------------------ euler_rows
 template <typename T>
