@@ -25,7 +25,8 @@ namespace dtb {
 
 struct MixedGroup {
     int in1 = 0, in2 = 0;
-    int M = 0, N1 = 0, n2 = 0, n2p = 0, n_cb = 0;
+    int M = 0, N1 = 0, n2 = 0, n2p = 0, n_cb = 0;  // M: stacked rows, each member's padded to 4
+    int rows = 0;                                  // stacked rows without the padding
     std::vector<std::pair<int, int>> members;  // (output species, first stacked row)
     unsigned char* gt = nullptr;  // G tiles [m_tiles][T][hi, lo][128 x 128 B], pre-swizzled
     float* row_scale = nullptr;
@@ -166,7 +167,7 @@ std::string g_plan_file;
 
 std::string plan_key(const dtb_ctx* c, const MixedGroup& G, int Bcols) {
     char k[160];
-    std::snprintf(k, sizeof(k), "sm%d:M%d:N1%d:n2%d:cols%d:cells%d", c->num_sms, G.M, G.N1, G.n2, Bcols,
+    std::snprintf(k, sizeof(k), "sm%d:M%d:N1%d:n2%d:cols%d:cells%d", c->num_sms, G.rows, G.N1, G.n2, Bcols,
                   (int)c->n_space);
     return k;
 }
@@ -445,8 +446,21 @@ int commit_mixed(dtb_ctx* c) {
             m->groups.push_back(G);
         }
         MixedGroup& G = m->groups[(size_t)gidx[key]];
-        G.members.push_back({g.out, G.M});
-        G.M += (int)c->sz[g.out];
+        G.members.push_back({g.out, G.rows});
+        G.rows += (int)c->sz[g.out];
+    }
+    // Members start on multiples of 4 rows, so that the epilogue gathers the split partials with
+    // 16-byte loads, where the padding takes no further 128-row tile of the GEMM.
+    for (auto& G : m->groups) {
+        int M = 0;
+        for (auto& mb : G.members) M += (int)round_up(c->sz[mb.first], 4);
+        G.M = G.rows;
+        if ((M + kMmaM - 1) / kMmaM != (G.rows + kMmaM - 1) / kMmaM) continue;
+        G.M = 0;
+        for (auto& mb : G.members) {
+            mb.second = G.M;
+            G.M += (int)round_up(c->sz[mb.first], 4);
+        }
     }
     DTB_CHECK(m->groups.size() <= 16, DTB_EINVAL, "at most 16 input pairs in a batched context");
     c->has_bin = !c->gains.empty() || !c->losses.empty();
@@ -503,8 +517,8 @@ int commit_mixed(dtb_ctx* c) {
     }
     for (auto& G : m->groups) {
         G.m_tiles = (G.M + kMmaM - 1) / kMmaM;
-        G.flops = 3.0 * 2.0 * G.M * (double)G.N1 * G.n2 * m->Buser * nsp;
-        G.bytes = 4.0 * G.M * (double)G.N1 * G.n2;
+        G.flops = 3.0 * 2.0 * G.rows * (double)G.N1 * G.n2 * m->Buser * nsp;
+        G.bytes = 4.0 * G.rows * (double)G.N1 * G.n2;
     }
     // ---------------- gain lookup per species
     {
@@ -763,35 +777,56 @@ int commit_mixed(dtb_ctx* c) {
         ops.grp_sig1[gi] = m->sig + (size_t)G.in1 * B;
         ops.grp_sig2[gi] = m->sig + (size_t)G.in2 * B;
     }
-    // tiles whose rows share one species and one list of emission pieces that cover all of
-    // them take the shared-memory tile products
+    // Row tiles: consecutive rows of one species and cell. Loss and emission run as tile products
+    // where every row of the tile has the same list of emission pieces, so a tile also ends where
+    // that list changes (not before its eighth row: shorter pieces keep the direct products).
     {
-        const int tr = mixed_rows_tile_rows();
-        const int n_tiles_r = (n_st + tr - 1) / tr;
         std::vector<std::vector<int>> emi_rows((size_t)n_st);
         for (size_t p = 0; p < c->emis.size(); ++p)
             for (int64_t r = 0; r < c->emis[p].nrows; ++r) emi_rows[(size_t)(c->emis[p].row0 + r)].push_back((int)p);
-        std::vector<unsigned char> fast((size_t)n_tiles_r, 1);
-        for (int t = 0; t < n_tiles_r; ++t) {
-            const int a0 = t * tr, a1 = std::min(n_st, a0 + tr);
-            const int s0 = species_of(c, a0 % n_mom);
-            if (a0 / n_mom != (a1 - 1) / n_mom) fast[(size_t)t] = 0;  // the tile lies in one cell
-            for (int a = a0; a < a1; ++a)
-                if (species_of(c, a % n_mom) != s0 || emi_rows[(size_t)a] != emi_rows[(size_t)a0]) fast[(size_t)t] = 0;
-            // and whose K chunks fit the kernel's job list
-            int64_t jobs = 0;
-            for (auto& kv : c->losses)
-                if (kv.first.first == s0) jobs += (c->sz[kv.first.second] + kRowsChunk - 1) / kRowsChunk;
-            for (int p : emi_rows[(size_t)a0]) jobs += (c->emis[(size_t)p].ncols + kRowsChunk - 1) / kRowsChunk;
-            if (jobs > kRowsMaxJobs) fast[(size_t)t] = 0;
+        const auto make_tiles = [&](int dim) {
+            std::vector<RowTile> tl;
+            for (int cell = 0; cell < nsp; ++cell)
+                for (int sp = 0; sp < c->ns; ++sp) {
+                    const int lo = cell * n_mom + (int)c->off[sp], hi = cell * n_mom + (int)c->off[sp + 1];
+                    for (int a0 = lo; a0 < hi;) {
+                        int end = std::min(hi, a0 + dim), fast = 1;
+                        for (int a = a0 + 1; a < end; ++a)
+                            if (emi_rows[(size_t)a] != emi_rows[(size_t)a0]) {
+                                if (a - a0 >= 8)
+                                    end = a;
+                                else
+                                    fast = 0;
+                                break;
+                            }
+                        // the K chunks must fit the kernel's job list
+                        int64_t jobs = 0;
+                        for (auto& kv : c->losses)
+                            if (kv.first.first == sp) jobs += (c->sz[kv.first.second] + kRowsChunk - 1) / kRowsChunk;
+                        for (int p : emi_rows[(size_t)a0])
+                            jobs += (c->emis[(size_t)p].ncols + kRowsChunk - 1) / kRowsChunk;
+                        if (jobs > kRowsMaxJobs) fast = 0;
+                        tl.push_back({a0, end - a0, cell, sp, 0, fast});
+                        a0 = end;
+                    }
+                }
+            return tl;
+        };
+        // 16 x 16 tiles where 32 x 32 ones leave half of the SMs without a block: four times the
+        // blocks, each with a quarter of the partials to gather. Steps of 256 instances on 2 x 128
+        // states (64 blocks of 32 x 32): 20.9 against 23.9 us; 21 instances on 3 x 258 states (27):
+        // 17.7 against 21.8 us; 256 on 2 x 256 (128): 58.8 against 55.9 us; 64 on 3 x 576 (108):
+        // 949 against 943 us.
+        ops.tile_dim = 32;
+        std::vector<RowTile> tiles = make_tiles(32);
+        if (2 * (int64_t)tiles.size() * ((B + 31) / 32) < c->num_sms) {
+            ops.tile_dim = 16;
+            tiles = make_tiles(16);
         }
-        unsigned char* d_fast;
-        DTB_TRY(copy_host_ints(c, &d_fast, fast));
-        ops.tile_fast = d_fast;
+        const int n_tiles_r = ops.n_tiles = (int)tiles.size();
         // the fast tiles' product chunks, in the layout of the loss and emission data above:
         // the loss blocks of the tile's species, then the emission pieces of its rows
         std::vector<RowJob> jobs((size_t)n_tiles_r * kRowsMaxJobs);
-        std::vector<int> njobs((size_t)n_tiles_r, 0);
         struct Opnd {
             const __nv_bfloat16* T;  // hi half of row 0 of the operand block, column 0
             int ld, col0, nc;
@@ -816,8 +851,8 @@ int commit_mixed(dtb_ctx* c) {
             }
         }
         for (int t = 0; t < n_tiles_r; ++t) {
-            if (!fast[(size_t)t]) continue;
-            const int a0 = t * tr, cell = a0 / n_mom, s0 = species_of(c, a0 % n_mom);
+            if (!tiles[(size_t)t].fast) continue;
+            const int a0 = tiles[(size_t)t].a0, cell = tiles[(size_t)t].cell, s0 = tiles[(size_t)t].sp;
             // the tile's operands at its first row: loss blocks read the tile's cell, emission
             // pieces their global columns; a loss block and an emission piece over the same state
             // rows share jobs
@@ -847,14 +882,14 @@ int commit_mixed(dtb_ctx* c) {
                 for (int c0 = 0; c0 < E[q].nc; c0 += kRowsChunk)
                     J[k++] = {nullptr, E[q].T, 0, E[q].ld, E[q].col0, E[q].nc, c0, 0};
             }
-            njobs[(size_t)t] = k;
+            tiles[(size_t)t].njobs = k;
         }
         RowJob* d_jobs;
-        int* d_nj;
+        RowTile* d_tiles;
         DTB_TRY(copy_host_ints(c, &d_jobs, jobs));
-        DTB_TRY(copy_host_ints(c, &d_nj, njobs));
+        DTB_TRY(copy_host_ints(c, &d_tiles, tiles));
         ops.jobs = d_jobs;
-        ops.njobs = d_nj;
+        ops.tiles = d_tiles;
     }
     ops.thr = (double)1e-10f;
     ops.has_bin = c->has_bin;
@@ -1081,7 +1116,7 @@ std::string batch_profile_json(const dtb_ctx* c) {
         const MixedGroup& G = m->groups[i];
         char b[160];
         std::snprintf(b, sizeof(b), "%s{\"M\": %d, \"pair\": %d, \"bn\": %d, \"n_splits\": %d, \"tuned_us\": %.4g}",
-                      i ? ", " : "", G.M, G.pair ? 1 : 0, G.bn, G.n_splits, G.tuned_us);
+                      i ? ", " : "", G.rows, G.pair ? 1 : 0, G.bn, G.n_splits, G.tuned_us);
         js += b;
     }
     return js + "]";

@@ -59,7 +59,7 @@ constexpr int kRowsChunk = 128;
 
 // One K chunk of an epilogue tile product: kRowsChunk columns of a row-major operand (loss or
 // emission rows, stored as BF16 hi and lo halves of the row-scaled values) against the same state
-// rows of the tile's instances. Built on the host per 32-row tile.
+// rows of the tile's instances. Built on the host per row tile.
 struct RowJob {
     const __nv_bfloat16* TL;  // loss operand (hi half) at the tile's first row, column 0, or null;
                               // the lo half is ops.loss_lo elements further
@@ -71,6 +71,13 @@ struct RowJob {
     int nc;           // operand columns
     int c0;           // first column of the chunk
     int pad;
+};
+
+// A tile of consecutive state rows of one species and cell.
+struct RowTile {
+    int a0, rows;     // first state row, rows (at most the tile height)
+    int cell, sp;
+    int njobs, fast;  // fast: loss and emission run as tile products, njobs chunks of them
 };
 
 // Per-row operands of the batched Euler epilogue.
@@ -117,9 +124,9 @@ struct MixedRowOps {
     const float* grp_rscale[16];
     const float* grp_sig1[16];    // [Bcap] power-of-two scale of input 1 per slot
     const float* grp_sig2[16];
-    const unsigned char* tile_fast;  // per 32-row tile: loss/emission as shared-memory tile products
+    int tile_dim, n_tiles;           // tile height and width (32 or 16); row tiles
+    const RowTile* tiles;            // [n_tiles]
     const RowJob* jobs;              // [tile][kRowsMaxJobs] product chunks of the fast tiles
-    const int* njobs;                // [tile]
     const float* invAp;
     const float* inj;
     double thr;
@@ -156,7 +163,6 @@ cudaError_t launch_admit_slot(const unsigned char* rec, int n, int ns, int slot,
                               int* nonfinite, unsigned long long inf_enc, cudaStream_t s);
 cudaError_t launch_pack_f(const double* io, int Buser, int n, int Bcap, float* F, float* C, cudaStream_t s);
 cudaError_t launch_unpack_f(const float* F, const float* C, int Buser, int n, int Bcap, double* io, cudaStream_t s);
-int mixed_rows_tile_rows();
 cudaError_t prepare_mixed_rows();
 
 cudaError_t launch_batch_moments(const float* F, const float* C, int Bcap, const int* sp_off, int n_species,

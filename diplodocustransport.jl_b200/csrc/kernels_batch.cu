@@ -7,7 +7,7 @@
 // Per 16-wide K step three MMAs accumulate hi*hi + hi*lo + lo*hi. One elected thread issues
 // the MMAs and commits them to mbarriers; every wait is bounded.
 //
-// mixed_rows: one (32 rows x 32 instances) tile per block: loss and emission (operands stored
+// mixed_rows: one tile of 32 rows x 32 instances (or 16 x 16) per block: loss and emission (operands stored
 // as BF16 hi+lo with per-row scales) as tensor-core tile products, split-K partial sums of the
 // gain, banded flux, then the update of SteppingMethods.jl:46-101 with an FP64 compensated
 // (Kahan) accumulation of f.
@@ -802,23 +802,27 @@ cudaError_t launch_split_rows(const float* src, long long rows, int row0, int n1
 namespace {
 
 
-constexpr int kRT = 32;   // rows per tile
-constexpr int kIT = 32;   // instances per tile
 constexpr int kCK = kRowsChunk;  // K chunk of the loss / emission tile products
 constexpr int kOP = kCK + 8;      // BF16 row pitch of a staged operand chunk (272 bytes: 16-byte
                                   // aligned rows whose 8-row ldmatrix phases hit 32 distinct banks)
-constexpr int kFP = kIT + 4;      // FP32 row pitch of a staged state chunk (conflict-free B loads)
 constexpr int kRowStages = 3;     // cp.async ring depth
-constexpr int kOpBytes = kRT * kOP * 2;  // one half (hi or lo) of one operand chunk
-constexpr int kStageBytes = 4 * kOpBytes + kCK * kFP * 4;  // loss hi, lo, emission hi, lo, state chunk
-constexpr int kRowsSmem = kRowStages * kStageBytes;  // dynamic: the operand / state chunk ring
+constexpr int kEllFast = 8;       // ELL widths up to this take the hoisted-load flux path
+constexpr int kGatherVec = 18;    // 16-byte split partials in flight per thread in the gain gather
 
-
-__device__ __forceinline__ int species_of_row(const MixedRowOps& ops, int a) {
-    int s = 0;
-    while (s + 1 < ops.n_species && a >= ops.sp_off[s + 1]) ++s;
-    return s;
-}
+// A tile of RT rows x IT instances on NW warps.
+template <int RT, int IT, int NW>
+struct RowsCfg {
+    static constexpr int TH = NW * 32;
+    static constexpr int NI = RT * IT / TH;              // instances a thread updates
+    static constexpr int KH = NW / ((RT / 16) * (IT / 8));  // K parts of each product chunk
+    static constexpr int NP = TH / (RT / 4 * IT);        // parts of the split range in the gain gather
+    static constexpr int FP = IT + 4;                    // FP32 row pitch of a staged state chunk (conflict-free B loads)
+    static constexpr int OPB = RT * kOP * 2;             // one half (hi or lo) of one operand chunk
+    static constexpr int STAGE = 4 * OPB + kCK * FP * 4; // loss hi, lo, emission hi, lo, state chunk
+    static constexpr int SMEM = kRowStages * STAGE;      // dynamic: the operand / state chunk ring
+    static_assert(NI >= 1 && NI <= 2 && NP >= 1 && KH >= 1 && kCK % (16 * KH) == 0, "tile shape");
+    static_assert((2 * KH + NP) * RT * (IT + 1) * 4 <= SMEM, "the parked sums fit the ring");
+};
 
 // Loss and emission of one (row, instance) pair with direct loads (tiles the fast path cannot take),
 // from the same BF16 hi + lo operands as the tile products: each operand value hi + lo (exact in
@@ -861,69 +865,68 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// One 32-row x 32-instance tile per block, 512 threads. Loss and emission are tile products
-// when the tile's rows belong to one species and every emission piece touching them covers
-// them all (tile_fast): all their K chunks form one job list streamed through a 3-stage
-// cp.async ring (operand chunk 32 x 128 as BF16 hi and lo halves, state chunk 128 x 32 FP32).
-// The products run on the tensor cores as m16n8k16 BF16 MMAs with FP32 accumulation: each of
-// the 16 warps owns a 16-row x 8-instance block over one half of every chunk's K range, splits
-// the state into BF16 hi + lo as it builds its B fragments, and accumulates
-// hi*hi + hi*lo + lo*hi (the scheme of the gain GEMM); the two K halves' sums are added in a
-// fixed order and scaled back by the rows' power-of-two scales. The update then gives each
-// thread one row and two instances, with every load it needs issued before the arithmetic
-// (flux columns and values, state, vectors), so the latency of the L2 round trips overlaps.
-constexpr int kRowsThreads = 512;
-constexpr int kKHalves = 2;  // K halves of each product chunk (8 warps each)
-static_assert(kRowsThreads / 32 == 2 * 4 * kKHalves, "16 warps: 2 row blocks x 4 instance blocks x 2 K halves");
-static_assert((2 * kKHalves + 2) * kRT * (kIT + 1) * 4 <= kRowStages * kStageBytes,
-              "the K halves' loss and emission tiles and the gather's half sums fit the ring");
-constexpr int kEllFast = 8;  // ELL widths up to this take the hoisted-load flux path
-constexpr int kGatherChunk = 18;  // split partials in flight per instance in the gain gather
-constexpr int kGatherVec = 18;    // 16-byte split partials in flight per thread in the vector gather
-
-__global__ void __launch_bounds__(kRowsThreads) mixed_rows_kernel(MixedRowOps ops, const float* __restrict__ F,
-                                                                  const float* __restrict__ Cc,
-                                                                  float* __restrict__ Fo, float* __restrict__ Co,
-                                                                  const unsigned long long* gstep, int kpos) {
-    __shared__ float s_gain[kRT][kIT + 1];
+// One tile of at most RT rows x IT instances per block. The rows of a tile belong to one species
+// of one cell. Loss and emission are tile products when every emission piece touching the tile's
+// rows covers them all (RowTile::fast): all their K chunks form one job list streamed through a
+// 3-stage cp.async ring (operand chunk RT x 128 as BF16 hi and lo halves, state chunk 128 x IT
+// FP32). The products run on the tensor cores as m16n8k16 BF16 MMAs with FP32 accumulation: each
+// warp owns a 16-row x 8-instance block over one of KH parts of every chunk's K range, splits the
+// state into BF16 hi + lo as it builds its B fragments, and accumulates hi*hi + hi*lo + lo*hi (the
+// scheme of the gain GEMM); the parts' sums are added in a fixed order and scaled back by the
+// rows' power-of-two scales. The update gives each thread one row and one or two instances, with
+// every load it needs issued before the arithmetic (flux columns and values, state, vectors, the
+// gain's scales), so the latency of the L2 round trips overlaps.
+template <int RT, int IT, int NW>
+__global__ void __launch_bounds__(NW * 32, 16 / NW) mixed_rows_kernel(MixedRowOps ops, const float* __restrict__ F,
+                                                                      const float* __restrict__ Cc,
+                                                                      float* __restrict__ Fo, float* __restrict__ Co,
+                                                                      const unsigned long long* gstep, int kpos) {
+    using K = RowsCfg<RT, IT, NW>;
+    constexpr int NI = K::NI, KH = K::KH, NP = K::NP, FP = K::FP, OPB = K::OPB, TH = K::TH;
     __shared__ RowJob s_job[kRowsMaxJobs];
-    __shared__ int s_njob;
     extern __shared__ __align__(16) float rows_dyn[];
-    // after the products the same memory holds the two K halves' loss and emission tiles
-    float(*s_pl)[kRT][kIT + 1] = reinterpret_cast<float(*)[kRT][kIT + 1]>(rows_dyn);
-    float(*s_pe)[kRT][kIT + 1] = reinterpret_cast<float(*)[kRT][kIT + 1]>(rows_dyn + kKHalves * kRT * (kIT + 1));
+    // after the products the same memory holds the K parts' loss and emission tiles
+    float(*s_pl)[RT][IT + 1] = reinterpret_cast<float(*)[RT][IT + 1]>(rows_dyn);
+    float(*s_pe)[RT][IT + 1] = reinterpret_cast<float(*)[RT][IT + 1]>(rows_dyn + KH * RT * (IT + 1));
+    float(*s_part)[RT][IT + 1] = reinterpret_cast<float(*)[RT][IT + 1]>(rows_dyn + 2 * KH * RT * (IT + 1));
     unsigned char* ring = reinterpret_cast<unsigned char*>(rows_dyn);
-    __shared__ double s_min[kRT][kIT + 1];  // padded: the per-instance reduction reads down columns
-    __shared__ int s_nonfin[kIT];
+    __shared__ double s_min[RT][IT + 1];  // padded: the per-instance reduction reads down columns
+    __shared__ int s_nonfin[IT];
     const int tid = threadIdx.x;
-    // products: warp w takes rows 16 (w & 1) .. + 15, instances 8 ((w >> 1) & 3) .. + 7 and the
-    // K half w >> 3 of every chunk
+    // products: warp w takes rows 16 (w mod RT/16) .. + 15, 8 instances and K part khalf of every chunk
     const int wp = tid >> 5, ln = tid & 31;
-    const int mblk = wp & 1, nblk = (wp >> 1) & 3, khalf = wp >> 3;
-    const int a0 = blockIdx.x * kRT, i0 = blockIdx.y * kIT;
-    const int n = ops.n_state, B = ops.Bcap;
+    const int mblk = wp % (RT / 16), nblk = wp / (RT / 16) % (IT / 8), khalf = wp / (RT / 16 * (IT / 8));
+    const RowTile tile = ops.tiles[blockIdx.x];
+    const int a0 = tile.a0, i0 = blockIdx.y * IT;
+    const int B = ops.Bcap;
     // the device step counter advances once per launch sequence (advance_step); kpos is this
     // launch's place in the sequence
     const long long step = (long long)*reinterpret_cast<const volatile unsigned long long*>(gstep) + kpos;
-    const bool fast = ops.tile_fast[blockIdx.x] != 0;
+    const bool fast = tile.fast != 0;
+    const int nj = tile.njobs;
 
-    if (fast) {  // the tile's product chunks (host-built job list)
-        if (tid < kRowsMaxJobs) s_job[tid] = ops.jobs[(size_t)blockIdx.x * kRowsMaxJobs + tid];
-        if (tid == 0) s_njob = ops.njobs[blockIdx.x];
-    }
+    // the tile's product chunks (host-built job list), in flight beside the tile's record
+    if (tid < kRowsMaxJobs) s_job[tid] = ops.jobs[(size_t)blockIdx.x * kRowsMaxJobs + tid];
     // ---- update operands, loaded ahead of the products so their latency overlaps them
-    const int r = tid >> 4;
+    const int r = tid / (IT / NI);
     const int a = a0 + r;
-    const int jb = (tid & 15) * 2;
+    const int jb = (tid % (IT / NI)) * NI;
     const int ib = i0 + jb;
-    const bool mine = a < n && ib < B;
+    const int am = a - tile.cell * ops.n_mom, s = tile.sp;
+    const bool mine = r < tile.rows && ib < B;
     const bool ell_fast = ops.ell_w <= kEllFast;
-    float2 fa2 = make_float2(0.f, 0.f), ca2 = make_float2(0.f, 0.f);
+    float fa[NI], ca[NI];
     double inv_ap = 0.0, injv = 0.0;
-    bool act[2] = {false, false};
-    double dts[2] = {0.0, 0.0};
+    bool act[NI];
+    double dts[NI];
     int cols[kEllFast];
     float vals[kEllFast];
+#pragma unroll
+    for (int j = 0; j < NI; ++j) {
+        fa[j] = ca[j] = 0.f;
+        act[j] = false;
+        dts[j] = 0.0;
+    }
 #pragma unroll
     for (int e = 0; e < kEllFast; ++e) {
         cols[e] = -1;
@@ -933,10 +936,10 @@ __global__ void __launch_bounds__(kRowsThreads) mixed_rows_kernel(MixedRowOps op
     if (mine) {
         inv_ap = (double)__ldg(ops.invAp + a);
         injv = (double)__ldg(ops.inj + a);
-        if (ops.has_bin) lsc = __ldg(ops.loss_rscale + (a % ops.n_mom));
+        if (ops.has_bin) lsc = __ldg(ops.loss_rscale + am);
         if (ops.has_emi) esc = __ldg(ops.emi_rscale + a);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < NI; ++j) {
             const int i = ib + j;
             act[j] = i < B && step < ops.stop_step[i];
             dts[j] = i < B ? ops.dt_scale[i] : 0.0;
@@ -963,58 +966,76 @@ __global__ void __launch_bounds__(kRowsThreads) mixed_rows_kernel(MixedRowOps op
     // the next step's GEMM may launch now: it waits for this grid's completion before it reads
     // the new state, so only its set-up (barriers, tensor memory, its first G tile) overlaps
     if (tid == 0) pdl_trigger();
-    // a chunk into ring stage st: 512 16-byte pieces of each operand half (32 rows x 128 BF16)
-    // and 1024 of the state (128 rows x 32 FP32), 4 + 2 per thread
+    // a chunk into ring stage st: 16-byte pieces of each operand half (RT rows x 128 BF16) and of
+    // the state (128 rows x IT FP32); rows past the tile's last are zero
     auto issue = [&](int k, int st) {
-        unsigned char* base = ring + (size_t)st * kStageBytes;
+        unsigned char* base = ring + (size_t)st * K::STAGE;
         const RowJob J = s_job[k];
-        {
-            const int rr = tid >> 4, c8 = (tid & 15) * 8;
-            const bool ok = a0 + rr < n && J.c0 + c8 < J.nc;
+#pragma unroll
+        for (int q = tid; q < RT * 16; q += TH) {
+            const int rr = q >> 4, c8 = (q & 15) * 8;
+            const bool ok = rr < tile.rows && J.c0 + c8 < J.nc;
             const size_t ol = (size_t)rr * kOP + c8;
             if (J.TL) {
                 const __nv_bfloat16* src = J.TL + (size_t)rr * J.ldl + J.c0 + c8;
                 cp_async16(base + 2 * ol, ok ? src : J.TL, ok ? 16 : 0);
-                cp_async16(base + kOpBytes + 2 * ol, ok ? src + ops.loss_lo : J.TL, ok ? 16 : 0);
+                cp_async16(base + OPB + 2 * ol, ok ? src + ops.loss_lo : J.TL, ok ? 16 : 0);
             }
             if (J.TE) {
                 const __nv_bfloat16* src = J.TE + (size_t)rr * J.lde + J.c0 + c8;
-                cp_async16(base + 2 * kOpBytes + 2 * ol, ok ? src : J.TE, ok ? 16 : 0);
-                cp_async16(base + 3 * kOpBytes + 2 * ol, ok ? src + ops.emi_lo : J.TE, ok ? 16 : 0);
+                cp_async16(base + 2 * OPB + 2 * ol, ok ? src : J.TE, ok ? 16 : 0);
+                cp_async16(base + 3 * OPB + 2 * ol, ok ? src + ops.emi_lo : J.TE, ok ? 16 : 0);
             }
         }
-        float* sF = reinterpret_cast<float*>(base + 4 * kOpBytes);
+        float* sF = reinterpret_cast<float*>(base + 4 * OPB);
 #pragma unroll
-        for (int q2 = 0; q2 < 2; ++q2) {
-            const int q = tid + kRowsThreads * q2;
-            const int cr = q >> 3, i4 = (q & 7) * 4;
+        for (int q = tid; q < kCK * (IT / 4); q += TH) {
+            const int cr = q / (IT / 4), i4 = (q % (IT / 4)) * 4;
             // state rows past the operand's columns are zero: the A operand there is zero too,
             // and zero times a stale value could be a NaN
             const bool okf = J.c0 + cr < J.nc && i0 + i4 < B;
             const float* srcf = okf ? F + (size_t)(J.col0 + J.c0 + cr) * B + i0 + i4 : F;
-            cp_async16(sF + cr * kFP + i4, srcf, okf ? 16 : 0);
+            cp_async16(sF + cr * FP + i4, srcf, okf ? 16 : 0);
         }
     };
     // the first chunks are in flight while the update's operands are loaded below
     if (fast) {
 #pragma unroll
         for (int k = 0; k < kRowStages - 1; ++k) {
-            if (k < s_njob) issue(k, k);
+            if (k < nj) issue(k, k);
             cp_async_commit();  // empty groups keep the group count uniform
         }
     }
+    const size_t idx = (size_t)a * B + ib;  // NI = 2: B and ib are even
     if (mine) {
-        const size_t idx = (size_t)a * B + ib;  // B and ib are even
-        fa2 = *reinterpret_cast<const float2*>(F + idx);
-        ca2 = *reinterpret_cast<const float2*>(Cc + idx);
+        if constexpr (NI == 2) {
+            const float2 f2 = *reinterpret_cast<const float2*>(F + idx), c2 = *reinterpret_cast<const float2*>(Cc + idx);
+            fa[0] = f2.x;
+            fa[1] = f2.y;
+            ca[0] = c2.x;
+            ca[1] = c2.y;
+        } else {
+            fa[0] = F[idx];
+            ca[0] = Cc[idx];
+        }
     }
-    if (tid < kIT) s_nonfin[tid] = 0;
+    if (tid < IT) s_nonfin[tid] = 0;
     __syncthreads();
-    float2 fv[kEllFast];
+    float fv[kEllFast][NI];
 #pragma unroll
-    for (int e = 0; e < kEllFast; ++e)
-        fv[e] = (mine && cols[e] >= 0) ? *reinterpret_cast<const float2*>(F + (size_t)cols[e] * B + ib)
-                                       : make_float2(0.f, 0.f);
+    for (int e = 0; e < kEllFast; ++e) {
+#pragma unroll
+        for (int j = 0; j < NI; ++j) fv[e][j] = 0.f;
+        if (mine && cols[e] >= 0) {
+            if constexpr (NI == 2) {
+                const float2 v2 = *reinterpret_cast<const float2*>(F + (size_t)cols[e] * B + ib);
+                fv[e][0] = v2.x;
+                fv[e][1] = v2.y;
+            } else {
+                fv[e][0] = F[(size_t)cols[e] * B + ib];
+            }
+        }
+    }
 
     // MMA accumulators of the warp's 16 x 8 block: rows g and g + 8, instances 2t and 2t + 1
     // (g = lane / 4, t = lane % 4)
@@ -1022,7 +1043,6 @@ __global__ void __launch_bounds__(kRowsThreads) mixed_rows_kernel(MixedRowOps op
     float acc_l[4] = {0.f, 0.f, 0.f, 0.f}, acc_e[4] = {0.f, 0.f, 0.f, 0.f};
     float cor_l[4] = {0.f, 0.f, 0.f, 0.f}, cor_e[4] = {0.f, 0.f, 0.f, 0.f};
     if (fast) {
-        const int nj = s_njob;
         const int g = ln >> 2, t = ln & 3;
         // ldmatrix row of this lane: matrices 0/1 take rows 0-7 / 8-15 at K 0-7, 2/3 at K 8-15
         const int lrow = 16 * mblk + (ln & 7) + ((ln >> 3) & 1) * 8, lcol = (ln >> 4) * 8;
@@ -1031,31 +1051,31 @@ __global__ void __launch_bounds__(kRowsThreads) mixed_rows_kernel(MixedRowOps op
             __syncthreads();  // chunk k landed for every thread; chunk k - 1's stage is free
             if (k + kRowStages - 1 < nj) issue(k + kRowStages - 1, (k + kRowStages - 1) % kRowStages);
             cp_async_commit();
-            const unsigned char* base = ring + (size_t)(k % kRowStages) * kStageBytes;
+            const unsigned char* base = ring + (size_t)(k % kRowStages) * K::STAGE;
             const uint32_t sa = smem_addr(base);
-            const float* sF = reinterpret_cast<const float*>(base + 4 * kOpBytes);
+            const float* sF = reinterpret_cast<const float*>(base + 4 * OPB);
             const bool hl = s_job[k].TL != nullptr, he = s_job[k].TE != nullptr;
 #pragma unroll
-            for (int kk = 0; kk < kCK / kKHalves / 16; ++kk) {
-                const int kb = khalf * (kCK / kKHalves) + kk * 16;
+            for (int kk = 0; kk < kCK / KH / 16; ++kk) {
+                const int kb = khalf * (kCK / KH) + kk * 16;
                 // B fragment: state rows kb + 2t, +1 and kb + 2t + 8, +9 of instance 8 nblk + g
-                const float* fp = sF + (kb + 2 * t) * kFP + 8 * nblk + g;
+                const float* fp = sF + (kb + 2 * t) * FP + 8 * nblk + g;
                 uint32_t bh0, bl0, bh1, bl1;
-                split_pair(fp[0], fp[kFP], bh0, bl0);
-                split_pair(fp[8 * kFP], fp[9 * kFP], bh1, bl1);
+                split_pair(fp[0], fp[FP], bh0, bl0);
+                split_pair(fp[8 * FP], fp[9 * FP], bh1, bl1);
                 const uint32_t ao = (uint32_t)(2 * (lrow * kOP + kb + lcol));
                 if (hl) {
                     uint32_t ah[4], al[4];
                     ldsm_x4(sa + ao, ah);
-                    ldsm_x4(sa + kOpBytes + ao, al);
+                    ldsm_x4(sa + OPB + ao, al);
                     mma_bf16_16816(acc_l, ah, bh0, bh1);
                     mma_bf16_16816(cor_l, ah, bl0, bl1);
                     mma_bf16_16816(cor_l, al, bh0, bh1);
                 }
                 if (he) {
                     uint32_t ah[4], al[4];
-                    ldsm_x4(sa + 2 * kOpBytes + ao, ah);
-                    ldsm_x4(sa + 3 * kOpBytes + ao, al);
+                    ldsm_x4(sa + 2 * OPB + ao, ah);
+                    ldsm_x4(sa + 3 * OPB + ao, al);
                     mma_bf16_16816(acc_e, ah, bh0, bh1);
                     mma_bf16_16816(cor_e, ah, bl0, bl1);
                     mma_bf16_16816(cor_e, al, bh0, bh1);
@@ -1063,7 +1083,7 @@ __global__ void __launch_bounds__(kRowsThreads) mixed_rows_kernel(MixedRowOps op
             }
         }
         cp_async_wait<0>();
-        __syncthreads();  // the ring is free: park the K halves' sums
+        __syncthreads();  // the ring is free: park the K parts' sums
         const int r0 = 16 * mblk + g, c0 = 8 * nblk + 2 * t;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -1079,135 +1099,94 @@ __global__ void __launch_bounds__(kRowsThreads) mixed_rows_kernel(MixedRowOps op
         s_pe[khalf][r0 + 8][c0] = acc_e[2];
         s_pe[khalf][r0 + 8][c0 + 1] = acc_e[3];
     }
+    // the binary term of this cell (SteppingMethods.jl:369-380): zero outside BinM.Domain
+    const bool bin_here = ops.has_bin && (ops.bin_on == nullptr || ops.bin_on[tile.cell] != 0);
     pdl_wait();  // this step's gain GEMM has completed: its split partials are visible
-    // ---- gain of the tile from the reduced group sums
-    // Vector gather (tiles of one cell and species whose group rows start on a multiple of 4,
-    // in groups of M a multiple of 4): the two halves of the block take the two halves of the
-    // split range, each thread 4 consecutive rows of one instance with 16-byte loads, all of a
-    // half's loads in flight at once (the scalar gather below needs two L2 round trips); each
-    // half sums its splits in order, and the two half sums are added in a fixed order.
-    bool vec_gain = false;
-    if (ops.has_bin && fast) {
-        const int cell = a0 / ops.n_mom, am0 = a0 - cell * ops.n_mom;
-        const int s = species_of_row(ops, am0);
-        vec_gain = a0 + kRT <= n;
-        for (int e = ops.gain_ptr[s]; e < ops.gain_ptr[s + 1] && vec_gain; ++e) {
-            const int gi = ops.gain_grp[e];
-            vec_gain = ((ops.gain_roff[e] + am0 - ops.sp_off[s]) % 4 == 0) && (ops.grp_M[gi] % 4 == 0);
-        }
-    }
-    if (vec_gain) {
-        float(*s_half)[kRT][kIT + 1] =
-            reinterpret_cast<float(*)[kRT][kIT + 1]>(rows_dyn + 2 * kKHalves * kRT * (kIT + 1));
-        const int cell = a0 / ops.n_mom, am0 = a0 - cell * ops.n_mom;
-        const int s = species_of_row(ops, am0);
-        const bool on = ops.bin_on == nullptr || ops.bin_on[cell] != 0;
-        const int h = tid >> 8, q = tid & 255, rg = q & 7, il = q >> 3;  // rows 4 rg .. + 3, instance il
-        const bool okv = on && i0 + il < B;
-        // the combine below: thread (row r, instances il0 and il0 + 16)
-        const int r = tid & (kRT - 1), il0 = tid >> 5;
-        float g0 = 0.f, g1 = 0.f;
+    // ---- gain of the tile: NP parts of the block take NP parts of the split range, each thread 4
+    // consecutive rows of one instance (16-byte loads where the group's rows allow it), all of a
+    // part's loads in flight at once; each part sums its splits in order, and the parts are added
+    // in order.
+    float gain[NI];
+#pragma unroll
+    for (int j = 0; j < NI; ++j) gain[j] = 0.f;
+    if (bin_here && ops.gain_ptr[s] < ops.gain_ptr[s + 1]) {
+        const int h = tid / (RT / 4 * IT), q = tid % (RT / 4 * IT), rg = q % (RT / 4), il = q / (RT / 4);
+        const bool okv = i0 + il < B && 4 * rg < tile.rows;
         for (int e = ops.gain_ptr[s]; e < ops.gain_ptr[s + 1]; ++e) {
             const int gi = ops.gain_grp[e];
-            const int row0 = ops.gain_roff[e] + (am0 - ops.sp_off[s]);
+            const int row0 = ops.gain_roff[e] + (a0 - tile.cell * ops.n_mom - ops.sp_off[s]);
             const int Mg = ops.grp_M[gi];
             const int nsp = ops.grp_nsplit[gi];
-            const int sp_lo = h == 0 ? 0 : (nsp + 1) / 2, sp_hi = h == 0 ? (nsp + 1) / 2 : nsp;
-            const float* pp = ops.grp_partial[gi] + ((size_t)cell * B + i0 + il) * Mg + row0 + 4 * rg;
+            const int sp_lo = h * nsp / NP, sp_hi = (h + 1) * nsp / NP;
+            const float* pp = ops.grp_partial[gi] + ((size_t)tile.cell * B + i0 + il) * Mg + row0 + 4 * rg;
             const size_t st = (size_t)ops.grp_stride[gi];
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int c0 = sp_lo; c0 < sp_hi; c0 += kGatherVec) {
-                float4 v[kGatherVec];
+            if (okv && row0 % 4 == 0 && Mg % 4 == 0) {
+                for (int c0 = sp_lo; c0 < sp_hi; c0 += kGatherVec) {
+                    float4 v[kGatherVec];
 #pragma unroll
-                for (int k = 0; k < kGatherVec; ++k)
-                    v[k] = (okv && c0 + k < sp_hi) ? *reinterpret_cast<const float4*>(pp + (size_t)(c0 + k) * st)
-                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int k = 0; k < kGatherVec; ++k)
+                        v[k] = c0 + k < sp_hi ? *reinterpret_cast<const float4*>(pp + (size_t)(c0 + k) * st)
+                                              : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int k = 0; k < kGatherVec; ++k) {
-                    if (c0 + k < sp_hi) {
-                        acc.x += v[k].x;
-                        acc.y += v[k].y;
-                        acc.z += v[k].z;
-                        acc.w += v[k].w;
-                    }
-                }
-            }
-            s_half[h][4 * rg][il] = acc.x;
-            s_half[h][4 * rg + 1][il] = acc.y;
-            s_half[h][4 * rg + 2][il] = acc.z;
-            s_half[h][4 * rg + 3][il] = acc.w;
-            __syncthreads();
-            const float rs = ops.grp_rscale[gi][row0 + r];
-            if (on && i0 + il0 < B)
-                g0 += (s_half[0][r][il0] + s_half[1][r][il0]) * rs * ops.grp_sig1[gi][i0 + il0] * ops.grp_sig2[gi][i0 + il0];
-            if (on && i0 + il0 + 16 < B)
-                g1 += (s_half[0][r][il0 + 16] + s_half[1][r][il0 + 16]) * rs * ops.grp_sig1[gi][i0 + il0 + 16] *
-                      ops.grp_sig2[gi][i0 + il0 + 16];
-            __syncthreads();  // s_half is reused by the next group
-        }
-        s_gain[r][il0] = g0;
-        s_gain[r][il0 + 16] = g1;
-    } else if (ops.has_bin) {
-        const int r = tid & (kRT - 1);
-        const int a = a0 + r;
-        const int cell = a / ops.n_mom, am = a - cell * ops.n_mom;
-        const int s = a < n ? species_of_row(ops, am) : 0;
-        const bool on = a < n && (ops.bin_on == nullptr || ops.bin_on[cell] != 0);
-        // the thread's two instances il0 and il0 + 16; their partials are loaded kGatherChunk
-        // splits at a time for both instances at once (one L2 round trip per chunk), then summed
-        // in split order
-        const int il0 = tid >> 5;
-        const bool ok0 = on && i0 + il0 < B, ok1 = on && i0 + il0 + 16 < B;
-        float g0 = 0.f, g1 = 0.f;
-        if (ok0 || ok1) {
-            for (int e = ops.gain_ptr[s]; e < ops.gain_ptr[s + 1]; ++e) {
-                const int gi = ops.gain_grp[e];
-                const int row = ops.gain_roff[e] + (am - ops.sp_off[s]);
-                const int Mg = ops.grp_M[gi];
-                // column cell * Bcap + slot of the group's partials
-                const float* pp0 = ops.grp_partial[gi] + ((size_t)cell * B + i0 + il0) * Mg + row;
-                const float* pp1 = pp0 + (size_t)16 * Mg;
-                const size_t st = (size_t)ops.grp_stride[gi];
-                const int nsp = ops.grp_nsplit[gi];
-                float acc0 = 0.f, acc1 = 0.f;
-                for (int sp0 = 0; sp0 < nsp; sp0 += kGatherChunk) {
-                    float v0[kGatherChunk], v1[kGatherChunk];
-#pragma unroll
-                    for (int k = 0; k < kGatherChunk; ++k) {
-                        const bool in = sp0 + k < nsp;
-                        v0[k] = (in && ok0) ? pp0[(size_t)(sp0 + k) * st] : 0.f;
-                        v1[k] = (in && ok1) ? pp1[(size_t)(sp0 + k) * st] : 0.f;
-                    }
-#pragma unroll
-                    for (int k = 0; k < kGatherChunk; ++k) {
-                        if (sp0 + k < nsp) {
-                            acc0 += v0[k];
-                            acc1 += v1[k];
+                    for (int k = 0; k < kGatherVec; ++k) {
+                        if (c0 + k < sp_hi) {
+                            acc.x += v[k].x;
+                            acc.y += v[k].y;
+                            acc.z += v[k].z;
+                            acc.w += v[k].w;
                         }
                     }
                 }
-                const float rs = ops.grp_rscale[gi][row];
-                if (ok0) g0 += acc0 * rs * ops.grp_sig1[gi][i0 + il0] * ops.grp_sig2[gi][i0 + il0];
-                if (ok1) g1 += acc1 * rs * ops.grp_sig1[gi][i0 + il0 + 16] * ops.grp_sig2[gi][i0 + il0 + 16];
+            } else if (okv) {
+                const int nr = min(4, Mg - (row0 + 4 * rg));
+                for (int c = sp_lo; c < sp_hi; ++c) {
+                    const float* p = pp + (size_t)c * st;
+                    acc.x += p[0];
+                    if (nr > 1) acc.y += p[1];
+                    if (nr > 2) acc.z += p[2];
+                    if (nr > 3) acc.w += p[3];
+                }
             }
+            s_part[h][4 * rg][il] = acc.x;
+            s_part[h][4 * rg + 1][il] = acc.y;
+            s_part[h][4 * rg + 2][il] = acc.z;
+            s_part[h][4 * rg + 3][il] = acc.w;
+            __syncthreads();
+            if (mine) {
+                const float rs = ops.grp_rscale[gi][row0 + r];
+#pragma unroll
+                for (int j = 0; j < NI; ++j) {
+                    float v = s_part[0][r][jb + j];
+#pragma unroll
+                    for (int p = 1; p < NP; ++p) v += s_part[p][r][jb + j];
+                    if (ib + j < B) gain[j] += v * rs * ops.grp_sig1[gi][ib + j] * ops.grp_sig2[gi][ib + j];
+                }
+            }
+            if (e + 1 < ops.gain_ptr[s + 1]) __syncthreads();  // s_part is reused by the next group
         }
-        s_gain[r][il0] = g0;
-        s_gain[r][il0 + 16] = g1;
+    } else {
+        __syncthreads();  // the parked products
     }
-    __syncthreads();
 
-    // ---- update: one row, two instances per thread
-    double rmin[2] = {CUDART_INF, CUDART_INF};
-    int nonfin[2] = {0, 0};
+    // ---- update: one row, NI instances per thread
+    double rmin[NI];
+    int nonfin[NI];
+#pragma unroll
+    for (int j = 0; j < NI; ++j) {
+        rmin[j] = CUDART_INF;
+        nonfin[j] = 0;
+    }
     if (mine) {
-        const size_t idx = (size_t)a * B + ib;
-        float flux[2] = {0.f, 0.f};
+        float flux[NI];
+#pragma unroll
+        for (int j = 0; j < NI; ++j) flux[j] = 0.f;
         if (ell_fast) {
 #pragma unroll
             for (int e = 0; e < kEllFast; ++e) {
                 if (cols[e] < 0) continue;  // padding: only stored entries take part
-                flux[0] += vals[e] * fv[e].x;
-                flux[1] += vals[e] * fv[e].y;
+#pragma unroll
+                for (int j = 0; j < NI; ++j) flux[j] += vals[e] * fv[e][j];
             }
         } else {
             const int* crow = ops.ell_col + (size_t)a * ops.ell_w;
@@ -1216,39 +1195,38 @@ __global__ void __launch_bounds__(kRowsThreads) mixed_rows_kernel(MixedRowOps op
                 const int col = __ldg(crow + e);
                 if (col < 0) continue;
                 const float v = __ldg(vrow + e);
-                const float2 f2 = *reinterpret_cast<const float2*>(F + (size_t)col * B + ib);
-                flux[0] += v * f2.x;
-                flux[1] += v * f2.y;
+#pragma unroll
+                for (int j = 0; j < NI; ++j)
+                    if (ib + j < B) flux[j] += v * F[(size_t)col * B + ib + j];
             }
         }
-        const int cell = a / ops.n_mom, am = a - cell * ops.n_mom;
-        const int s = species_of_row(ops, am);
-        // the binary term of this cell (SteppingMethods.jl:369-380): Vol of the cell, zero outside
-        // BinM.Domain
-        const bool bin_here = ops.has_bin && (ops.bin_on == nullptr || ops.bin_on[cell] != 0);
-        const float vol = ops.vol_cell[cell];
-        const float fa[2] = {fa2.x, fa2.y};
-        const float ca[2] = {ca2.x, ca2.y};
-        float fo[2], co[2];
+        const float vol = ops.vol_cell[tile.cell];
+        float fo[NI], co[NI];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < NI; ++j) {
             if (!act[j]) {
                 fo[j] = fa[j];
                 co[j] = ca[j];
                 continue;
             }
             float loss, emi;
-            if (fast) {  // the K halves in a fixed order, then the rows' scales (powers of two)
-                loss = (s_pl[0][r][jb + j] + s_pl[1][r][jb + j]) * lsc;
-                emi = (s_pe[0][r][jb + j] + s_pe[1][r][jb + j]) * esc;
+            if (fast) {  // the K parts in a fixed order, then the rows' scales (powers of two)
+                loss = s_pl[0][r][jb + j];
+                emi = s_pe[0][r][jb + j];
+#pragma unroll
+                for (int p = 1; p < KH; ++p) {
+                    loss += s_pl[p][r][jb + j];
+                    emi += s_pe[p][r][jb + j];
+                }
+                loss *= lsc;
+                emi *= esc;
             } else {
-                row_terms_direct(ops, F, a, am, cell, s, ib + j, loss, emi);
+                row_terms_direct(ops, F, a, am, tile.cell, s, ib + j, loss, emi);
             }
-            const float gain = ops.has_bin ? s_gain[r][jb + j] : 0.f;
             // SteppingMethods.jl:31-46 in FP32, the scaling in FP64
             float df = -flux[j];
             if (ops.has_emi) df += emi;
-            if (ops.has_bin) df += bin_here ? vol * (gain - fa[j] * loss) : 0.f;
+            if (ops.has_bin) df += bin_here ? vol * (gain[j] - fa[j] * loss) : 0.f;
             const double dfs = (double)df * (inv_ap * dts[j]);
             // :97-101 with an FP64 compensated sum: the state is fa + ca
             double t = ((double)fa[j] + (double)ca[j]) + (dfs + injv * dts[j]);
@@ -1261,24 +1239,34 @@ __global__ void __launch_bounds__(kRowsThreads) mixed_rows_kernel(MixedRowOps op
             if (ratio < rmin[j] || (ratio == rmin[j] && signbit(ratio))) rmin[j] = ratio;
             if (!isfinite(dfs)) nonfin[j] = 1;
         }
-        *reinterpret_cast<float2*>(Fo + idx) = make_float2(fo[0], fo[1]);
-        *reinterpret_cast<float2*>(Co + idx) = make_float2(co[0], co[1]);
+        if constexpr (NI == 2) {
+            *reinterpret_cast<float2*>(Fo + idx) = make_float2(fo[0], fo[1]);
+            *reinterpret_cast<float2*>(Co + idx) = make_float2(co[0], co[1]);
+        } else {
+            Fo[idx] = fo[0];
+            Co[idx] = co[0];
+        }
     }
     // ---- per-instance diagnostics over the tile's rows, then one atomic per instance
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < NI; ++j) {
         s_min[r][jb + j] = rmin[j];
         if (nonfin[j]) atomicOr(&s_nonfin[jb + j], 1);
     }
     __syncthreads();
     {
-        // 16 lanes per instance, two rows each, then a shuffle tree (min with -0.0 below +0.0)
-        const int il = tid >> 4, rg = tid & 15;
+        // TH / IT lanes per instance, RT / lanes rows each, then a shuffle tree (min with -0.0 below +0.0)
+        constexpr int L = TH / IT;
+        static_assert(L == 16 && RT % L == 0, "16 lanes per instance");
+        const int il = tid / L, rg = tid % L;
         double m = s_min[rg][il];
-        const double v2 = s_min[rg + 16][il];
-        if (v2 < m || (v2 == m && signbit(v2))) m = v2;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
+        for (int q = 1; q < RT / L; ++q) {
+            const double v2 = s_min[rg + q * L][il];
+            if (v2 < m || (v2 == m && signbit(v2))) m = v2;
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) {
             const double v = __shfl_xor_sync(0xffffffffu, m, o);
             if (v < m || (v == m && signbit(v))) m = v;
         }
@@ -1424,16 +1412,20 @@ cudaError_t launch_advance_step(unsigned long long* gstep, int n, cudaStream_t s
 
 cudaError_t launch_mixed_rows(const MixedRowOps& ops, const float* F_in, const float* C_in, float* F_out, float* C_out,
                               const unsigned long long* gstep, int kpos, cudaStream_t s) {
-    dim3 grid((ops.n_state + kRT - 1) / kRT, (ops.Bcap + kIT - 1) / kIT);
-    return launch_pdl(mixed_rows_kernel, grid, dim3(kRowsThreads), (size_t)kRowsSmem, s, ops, F_in, C_in, F_out, C_out,
-                      gstep, kpos);
+    const dim3 grid(ops.n_tiles, (ops.Bcap + ops.tile_dim - 1) / ops.tile_dim);
+    if (ops.tile_dim == 32)
+        return launch_pdl(mixed_rows_kernel<32, 32, 16>, grid, dim3(512), (size_t)RowsCfg<32, 32, 16>::SMEM, s, ops, F_in,
+                          C_in, F_out, C_out, gstep, kpos);
+    return launch_pdl(mixed_rows_kernel<16, 16, 8>, grid, dim3(256), (size_t)RowsCfg<16, 16, 8>::SMEM, s, ops, F_in, C_in,
+                      F_out, C_out, gstep, kpos);
 }
 
-
-int mixed_rows_tile_rows() { return kRT; }
-
 cudaError_t prepare_mixed_rows() {
-    return cudaFuncSetAttribute(mixed_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem);
+    cudaError_t e = cudaFuncSetAttribute(mixed_rows_kernel<32, 32, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         RowsCfg<32, 32, 16>::SMEM);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(mixed_rows_kernel<16, 16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                RowsCfg<16, 16, 8>::SMEM);
 }
 
 }  // namespace dtb
