@@ -211,6 +211,7 @@ void apply_plan(MixedGroup& G, const GemmPlan& p, int Bcols) {
 constexpr int kMaxTilesPerAccSm = 16;
 constexpr int kMaxTilesPerAccPair = 32;
 constexpr int kMaxWaves = 4;
+constexpr int kShortSplit = 16;  // K tiles: splits this short are also tried longer (tune_group)
 int fill_splits(const dtb_ctx* c, const MixedGroup& G, int pair, int bn, int Bcols, int max_pairs) {
     const int n_tiles = (Bcols + bn - 1) / bn;
     const double units = pair ? (double)(G.m_tiles / 2 * n_tiles) : (double)(G.m_tiles * n_tiles);
@@ -269,26 +270,46 @@ GemmArgs gemm_args(const dtb_ctx* c, const MixedGroup& G, const float* Fin) {
     return a;
 }
 
+// The epilogue's view of a group under its current plan.
+void set_group_ops(MixedRowOps& ops, const MixedGroup& G, int gi) {
+    ops.grp_partial[gi] = G.partial;
+    ops.grp_stride[gi] = (long long)G.Bpad * G.M;
+    ops.grp_nsplit[gi] = G.n_splits;
+    ops.grp_M[gi] = G.M;
+}
+
 cudaError_t launch_group_gemm(const dtb_ctx* c, const MixedGroup& G, const float* Fin) {
     const GemmArgs a = gemm_args(c, G, Fin);
     return G.pair ? launch_gain_gemm_pair(a, c->stream) : launch_gain_gemm(G.bn, a, c->stream);
 }
 
-// Times each candidate plan of one group on the device (every column running, the state at its
-// committed zeros: tensor-core time does not depend on the values) and returns the fastest.
+// Times each candidate plan of one group on the device, the GEMM followed by the epilogue over the
+// group (every column running, the state at its committed zeros: tensor-core time does not depend
+// on the values; no slot steps, so the epilogue gathers the partials and changes nothing), and
+// returns the fastest. The GEMM alone misleads: more splits mean more partials to gather, and a
+// GEMM that leaves SMs free lets the epilogue's products run beside it. So splits of at most
+// kShortSplit K tiles are also tried half as long again and twice as long. 256 instances on 2 x 128
+// states: 17.5 us per step with 128-wide tiles on one SM and 36 splits against 19.6 with the fastest
+// GEMM (SM pairs, 74 splits); 16 instances: 12.5 us with 50 splits against 14.9 with 74.
 int tune_group(dtb_ctx* c, MixedGroup& G, int Bcols, int max_pairs, GemmPlan* best) {
     MixedState* m = c->mixed;
     std::vector<GemmPlan> cands;
+    const int T = G.n_cb * G.N1;
     for (int bn : {64, 128, 256}) {
         if (bn > 64 && bn / 2 >= Bcols) continue;  // half the tile or more would be padding
-        GemmPlan p;
-        p.bn = bn;
-        p.splits = fill_splits(c, G, 0, bn, Bcols, max_pairs);
-        cands.push_back(p);
-        if (bn == 256 && G.m_tiles % 2 == 0 && max_pairs > 0) {
-            p.pair = 1;
-            p.splits = fill_splits(c, G, 1, bn, Bcols, max_pairs);
+        for (int pair : {0, 1}) {
+            if (pair && (bn != 256 || G.m_tiles % 2 != 0 || max_pairs <= 0)) continue;
+            GemmPlan p;
+            p.bn = bn;
+            p.pair = pair;
+            p.splits = fill_splits(c, G, pair, bn, Bcols, max_pairs);
             cands.push_back(p);
+            const int fill = p.splits;
+            if (T > kShortSplit * fill) continue;
+            for (int part : {2, 1}) {  // two thirds, half of the splits
+                p.splits = fill * part / (part + 1);
+                if (p.splits >= 1) cands.push_back(p);
+            }
         }
     }
     *best = heuristic_plan(c, G, Bcols, max_pairs);
@@ -316,6 +337,18 @@ int tune_group(dtb_ctx* c, MixedGroup& G, int Bcols, int max_pairs, GemmPlan* be
     DTB_CUDA(cudaEventCreate(&sc.e1));
     float* const part = sc.part;
     const cudaEvent_t e0 = sc.e0, e1 = sc.e1;
+    // the epilogue over this group alone
+    MixedRowOps ops = m->ops;
+    const int gi = (int)(&G - m->groups.data());
+    for (int sp = 0, e = 0; sp < c->ns; ++sp) {
+        ops.gain_ptr[sp] = e;
+        for (auto& mb : G.members)
+            if (mb.first == sp) {
+                ops.gain_grp[e] = gi;
+                ops.gain_roff[e++] = mb.second;
+            }
+        ops.gain_ptr[sp + 1] = e;
+    }
     const int all = Bcols;
     DTB_CUDA(cudaMemcpyAsync(m->active_hi, &all, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     double best_ms = 1e30;
@@ -323,24 +356,29 @@ int tune_group(dtb_ctx* c, MixedGroup& G, int Bcols, int max_pairs, GemmPlan* be
     for (const GemmPlan& p : cands) {
         apply_plan(G, p, Bcols);
         G.partial = part;
+        set_group_ops(ops, G, gi);
         constexpr int kWarm = 2, kRep = 5;
+        float ms[2] = {0, 0};  // per GEMM, per GEMM and epilogue
         cudaError_t e = cudaSuccess;
-        for (int k = 0; k < kWarm && e == cudaSuccess; ++k) e = launch_group_gemm(c, G, m->F[0]);
-        if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
-        for (int k = 0; k < kRep && e == cudaSuccess; ++k) e = launch_group_gemm(c, G, m->F[0]);
-        if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-        float ms = 0;
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+        for (int rows = 0; rows < 2 && e == cudaSuccess; ++rows) {
+            for (int k = 0; k < kWarm + kRep && e == cudaSuccess; ++k) {
+                if (k == kWarm) e = cudaEventRecord(e0, c->stream);
+                if (e == cudaSuccess) e = launch_group_gemm(c, G, m->F[0]);
+                if (e == cudaSuccess && rows)
+                    e = launch_mixed_rows(ops, m->F[0], m->C[0], m->F[1], m->C[1], m->gstep, 0, c->stream);
+            }
+            if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
+            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms[rows], e0, e1);
+        }
         if (e != cudaSuccess) {  // a plan this device cannot launch is skipped
             cudaGetLastError();
             continue;
         }
-        const double per = ms / kRep;
-        if (per < best_ms) {
-            best_ms = per;
+        if (ms[1] / kRep < best_ms) {
+            best_ms = ms[1] / kRep;
             *best = p;
-            best->us = per * 1e3;
+            best->us = ms[0] / kRep * 1e3;
         }
     }
     const int zero = 0;
@@ -759,8 +797,6 @@ int commit_mixed(dtb_ctx* c) {
     DTB_CUDA(cudaMallocHost(&c->pin_err, sizeof(int)));
     m->h_stop.assign((size_t)B, 0);
     m->h_start.assign((size_t)B, 0);
-    // ---------------- GEMM plan per group: tile width, kernel and K splits (autotuned)
-    DTB_TRY(plan_gemms(c, Bcols, max_pairs));
     ops.n_mom = n_mom;
     ops.n_state = n_st;
     ops.n_space = nsp;
@@ -769,10 +805,6 @@ int commit_mixed(dtb_ctx* c) {
     for (int sp = 0; sp <= c->ns; ++sp) ops.sp_off[sp] = (int)c->off[sp];
     for (size_t gi = 0; gi < m->groups.size(); ++gi) {
         const MixedGroup& G = m->groups[gi];
-        ops.grp_partial[gi] = G.partial;
-        ops.grp_stride[gi] = (long long)G.Bpad * G.M;
-        ops.grp_nsplit[gi] = G.n_splits;
-        ops.grp_M[gi] = G.M;
         ops.grp_rscale[gi] = G.row_scale;
         ops.grp_sig1[gi] = m->sig + (size_t)G.in1 * B;
         ops.grp_sig2[gi] = m->sig + (size_t)G.in2 * B;
@@ -898,6 +930,9 @@ int commit_mixed(dtb_ctx* c) {
     ops.stop_step = m->stop_step;
     ops.min_ratio = m->min_ratio;
     ops.nonfinite = m->nonfinite;
+    // ---------------- GEMM plan per group: tile width, kernel and K splits (autotuned)
+    DTB_TRY(plan_gemms(c, Bcols, max_pairs));
+    for (size_t gi = 0; gi < m->groups.size(); ++gi) set_group_ops(ops, m->groups[gi], (int)gi);
     for (auto& G : m->groups) c->gain_bytes += G.bytes;
     DTB_CUDA(cudaDeviceSynchronize());
     return DTB_OK;
