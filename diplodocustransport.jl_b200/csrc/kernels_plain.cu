@@ -21,127 +21,14 @@
 
 #include "dtb_internal.h"
 #include "pdl.cuh"
+#include "plain_step.cuh"
 
 namespace dtb {
 
-// ------------------------------------------------------------------ PTX helpers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ unsigned long long globaltimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Waits for the phase with the given parity; gives up after kWaitLimitNs or when another
-// role of the block raised the abort flag.
-__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const unsigned long long t0 = globaltimer();
-    while (true) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-        if (globaltimer() - t0 > kWaitLimitNs) return false;
-    }
-}
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-        "l"(src), "r"(bytes), "r"(bar)
-        : "memory");
-}
-template <typename T>
-__device__ __forceinline__ T warp_sum(T v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// Julia's min on Float64 with -0.0 ordered below +0.0 (NaN is mapped to Inf before).
-__device__ __forceinline__ double jl_min(double a, double b) {
-    if (a < b) return a;
-    if (b < a) return b;
-    return signbit(a) ? a : b;
-}
-__device__ __forceinline__ double nan_to_inf(double x) { return isnan(x) ? CUDART_INF : x; }
-
-// Julia `x * b::Bool` = ifelse(b, x, copysign(0, x)).
-template <typename T>
-__device__ __forceinline__ T jl_mul_bool(T x, bool b) {
-    return b ? x : copysign(T(0), x);
-}
-
 // ------------------------------------------------------------------ gain_stream
-struct SpOff {
-    int n;
-    int off[DTB_MAX_SPECIES + 1];   // unpadded
-    int offp[DTB_MAX_SPECIES + 1];  // padded (multiples of 8)
-};
-
-// 16 bytes of G as FP64 values.
-template <typename T>
-struct Vec;
-template <>
-struct Vec<float> {
-    using type = float4;
-    static constexpr int n = 4;
-    __device__ __forceinline__ static void unpack(const float4& g, double (&v)[4]) {
-        v[0] = g.x;
-        v[1] = g.y;
-        v[2] = g.z;
-        v[3] = g.w;
-    }
-};
-template <>
-struct Vec<double> {
-    using type = double2;
-    static constexpr int n = 2;
-    __device__ __forceinline__ static void unpack(const double2& g, double (&v)[2]) {
-        v[0] = g.x;
-        v[1] = g.y;
-    }
-};
-
-constexpr int kGainThreads = (kGainConsumerWarps + 1) * 32;
-constexpr int kGainConsumers = kGainConsumerWarps * 32;
-
-__host__ __device__ constexpr int round_up_int(int x, int m) { return (x + m - 1) / m * m; }
-__host__ __device__ constexpr int pow2_ceil(int x) { return x <= 1 ? 1 : 2 * pow2_ceil((x + 1) / 2); }
-
 // Reduction ring: a consumer warp can run at most kGainStages tiles (hence units) ahead of
 // warp 0, so kGainStages + 2 slots never alias a slot warp 0 is still reading.
 constexpr int kRedRing = kGainStages + 2;
-
-// Staged states: in the state type for one cell, FP64 for several (one conversion per state and
-// block, not one per b-row).
-template <typename T, int C>
-struct StagedT {
-    using type = double;
-};
-template <typename T>
-struct StagedT<T, 1> {
-    using type = T;
-};
 
 int gain_stream_smem_bytes(int elem_size, int f_smem_len, int cells) {
     return kGainStages * kGainTileBytes + round_up_int(f_smem_len * cells * (cells == 1 ? elem_size : 8), 16) +
@@ -149,128 +36,9 @@ int gain_stream_smem_bytes(int elem_size, int f_smem_len, int cells) {
            kRedRing * kGainConsumerWarps * cells * 8 + 16;
 }
 
-// Sums of N values over the warp's 32 lanes: halving exchanges while several values are left,
-// then a butterfly. Lane l of the result holds value l >> (5 - log2 N). Every value is summed by
-// the same tree (lane distances 16, 8, 4, 2, 1), so its bits do not depend on N.
-template <int N>
-__device__ __forceinline__ double warp_sum_n(double (&v)[N], int lane) {
-    int o = 16;
-#pragma unroll
-    for (int n = N; n > 1; n /= 2, o >>= 1) {
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int i = 0; i < N / 2; ++i) {
-            if (i < n / 2) {
-                const double send = up ? v[i] : v[i + n / 2];
-                const double keep = up ? v[i + n / 2] : v[i];
-                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-            }
-        }
-    }
-#pragma unroll
-    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-    return v[0];
-}
-
-// Thread `tid`'s share of one work unit: the 16-byte columns cv, cv + w, .. (KV of them, w threads
-// to a b-row) of b-rows r0, r0 + dr, .. of every tile.
-struct UnitMap {
-    int nvr, w, dr, r0, cv;
-    bool on;
-};
-template <typename T, int KV>
-__device__ __forceinline__ UnitMap unit_map(const GainUnit& U, int tid) {
-    UnitMap m;
-    m.nvr = U.n2p / Vec<T>::n;
-    m.w = (m.nvr + KV - 1) / KV;
-    m.dr = kGainConsumers / m.w;
-    m.r0 = tid / m.w;
-    m.cv = tid - m.r0 * m.w;
-    m.on = m.r0 < m.dr;
-    return m;
-}
-
-// y[kv][c][e] += f1[b][c] G[b][column kv, element e] over the thread's b-rows of one tile, in
-// order. FP64 throughout: with one cell that is 2 (FP64) or 4 (FP32) FMAs per 16 bytes, and one
-// broadcast read of f1 per row; with C cells the tile is read once for all of them.
-template <typename T, int C, int KV>
-__device__ __forceinline__ void tile_accumulate(const UnitMap& m, const unsigned char* tile, int rows,
-                                                const typename StagedT<T, C>::type* f1, int f_len,
-                                                double (&y)[KV][C][Vec<T>::n]) {
-    using V = Vec<T>;
-    using vec_t = typename V::type;
-    if (!m.on) return;
-    const vec_t* tv = reinterpret_cast<const vec_t*>(tile);
-    constexpr int kUnroll = KV * C * V::n <= 8 ? 2 : 1;
-#pragma unroll kUnroll
-    for (int r = m.r0; r < rows; r += m.dr) {
-        double g[KV][V::n];
-#pragma unroll
-        for (int k = 0; k < KV; ++k) {
-            // a column past the row's end repeats the last one; its sum is not used
-            const int cv = k == 0 ? m.cv : min(m.cv + k * m.w, m.nvr - 1);
-            V::unpack(tv[r * m.nvr + cv], g[k]);
-        }
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            const double x = (double)f1[c * f_len + r];
-#pragma unroll
-            for (int k = 0; k < KV; ++k)
-#pragma unroll
-                for (int e = 0; e < V::n; ++e) y[k][c][e] = fma(x, g[k][e], y[k][c][e]);
-        }
-    }
-}
-
-// The unit's contraction with f2 and the warp's sum; lane l holds cell l >> (5 - log2 pow2_ceil(C)).
-template <typename T, int C, int KV>
-__device__ __forceinline__ double unit_warp_sum(const UnitMap& m, const typename StagedT<T, C>::type* f2, int f_len,
-                                                double (&y)[KV][C][Vec<T>::n], int lane) {
-    using V = Vec<T>;
-    double acc[pow2_ceil(C)];
-#pragma unroll
-    for (int c = 0; c < pow2_ceil(C); ++c) acc[c] = 0.0;
-    if (m.on) {
-#pragma unroll
-        for (int k = 0; k < KV; ++k) {
-            if (k == 0 || m.cv + k * m.w < m.nvr) {
-                const typename StagedT<T, C>::type* x = f2 + (m.cv + k * m.w) * V::n;
-#pragma unroll
-                for (int c = 0; c < C; ++c)
-#pragma unroll
-                    for (int e = 0; e < V::n; ++e) acc[c] = fma((double)x[c * f_len + e], y[k][c][e], acc[c]);
-            }
-        }
-    }
-    return warp_sum_n<pow2_ceil(C)>(acc, lane);
-}
-
-// The cells of a pass, padded per species ([cell][state]: the lanes of a warp read consecutive
-// states of one cell); zeros in the padding and for cells past the last.
-template <typename T, int C>
-__device__ __forceinline__ void stage_f(typename StagedT<T, C>::type* f_s, const T* __restrict__ f, const SpOff& so,
-                                        int f_len, int n_mom, const int* cell_list, int cell0, int n_cells, int tid,
-                                        int n_threads) {
-    for (int i = tid; i < f_len; i += n_threads) {
-        int s = 0;
-        while (s + 1 < so.n && i >= so.offp[s + 1]) ++s;
-        const int j = i - so.offp[s];
-        const bool in = j < so.off[s + 1] - so.off[s];
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            T v = T(0);
-            if (in && cell0 + c < n_cells) {
-                const int cell = cell_list ? cell_list[cell0 + c] : cell0 + c;
-                v = f[(size_t)cell * n_mom + so.off[s] + j];
-            }
-            f_s[c * f_len + i] = v;
-        }
-    }
-}
-
 // One block streams work units through a ring of 16 KB tiles for up to C space cells at once
 // (grid y: groups of C cells), so G crosses HBM once per group and not once per cell. Bound: HBM
-// with one cell (2 x 1024 states in FP32: 6.5 TB/s, the copy rate); with eight FP64 cells the
+// with one cell (2 x 1024 states in FP32: 7.1 TB/s); with eight FP64 cells the
 // shared-memory reads and the work per 16 KB tile (4.8 TB/s of G on 2 x 256 states). At most 96
 // registers: two CTAs of nine warps per SM.
 template <typename T, int C, int KV>
@@ -368,13 +136,15 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
     asm volatile("bar.sync 1, %0;" ::"n"(kGainConsumers) : "memory");  // the consumer warps only
     uint32_t it = 0;
     uint32_t lk = 0;  // units done by this block
+    UnitSum<T, C, KV> sum;
+    int c_off = -1, n2p = 0;  // the columns in sum's x
     for (int u = blockIdx.x; u < n_units; u += gridDim.x, ++lk) {
         const int slot = lk % kRedRing;
         const GainUnit* U = &unit_s[slot];  // valid from the unit's first tile on
         UnitMap m{};
-        double y[KV][C][Vec<T>::n] = {};
         const S* f1 = f_s;
-        int left = 1, tile_b = 0;  // b-rows left; at least one tile
+        sum.begin();
+        int left = 1, tile_b = 0, r = 0;  // b-rows left (at least one tile), the thread's next b-row
         for (; left > 0; left -= tile_b, f1 += tile_b, ++it) {
             const int st = it % kGainStages;
             const uint32_t ph = (it / kGainStages) & 1u;
@@ -384,16 +154,26 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
                 return;
             }
             if (tile_b == 0) {
-                m = unit_map<T, KV>(*U, tid);
+                m = unit_map<T, KV>(U->n2p, tid);
+                r = m.r0;
+                if (sum.kDotRows && (U->c_off != c_off || U->n2p != n2p)) {
+                    c_off = U->c_off;
+                    n2p = U->n2p;
+                    sum.load_x(m, f_s + c_off, f_len);
+                }
                 f1 += U->b_off;
                 left = U->nb;
                 tile_b = U->tile_b;
             }
-            tile_accumulate<T, C, KV>(m, smem + (size_t)st * kGainTileBytes, min(tile_b, left), f1, f_len, y);
+            sum.tile(m, smem + (size_t)st * kGainTileBytes, min(tile_b, left), r, f1, f_len);
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&empty[st]));
         }
-        const double acc = unit_warp_sum<T, C, KV>(m, f_s + U->c_off, f_len, y, lane);
+        sum.finish(m, f_s + U->c_off, f_len);
+        double part[pow2_ceil(C)];
+#pragma unroll
+        for (int c = 0; c < pow2_ceil(C); ++c) part[c] = c < C ? sum.acc[c < C ? c : 0] : 0.0;
+        const double acc = warp_sum_n<pow2_ceil(C)>(part, lane);
         constexpr int kLanes = 32 / pow2_ceil(C);  // lanes per cell of the warp's sums
         if (lane % kLanes == 0 && lane / kLanes < C) red[(slot * kGainConsumerWarps + warp) * C + lane / kLanes] = acc;
         __syncwarp();
@@ -455,17 +235,21 @@ int pass_blocks_per_sm(const GainPass& p, int f_smem_len) {
 // at most) and the staged states a CTA's shared memory, split evenly over the passes they take
 // (the least padding). G is the traffic: eight cells of a 2 x 256-state FP64 grid (268 MB of G)
 // take 61 us per step in one pass and 321 us in eight.
-// 16-byte columns per thread: as many as cover the longest b-row with 256 threads. With three or
-// more FP64 cells at least two, since every cell costs a broadcast read of f1 per b-row and two
-// columns share it (one FP64 FMA pair per read is too little to hide it behind).
+// 16-byte columns per thread: what covers the longest b-row with 256 threads, and with three or more
+// FP64 cells at least two, since every cell costs a broadcast read of f1 per b-row and the columns
+// share it. One FP32 cell takes four where a b-row then still fills a warp: they also share f1's
+// conversion (77 against 85 ms for 64 steps of 2 x 1024 states). On shorter b-rows, and with FP64,
+// more columns cost more in idle threads than they save (40 steps of 2 x 128 FP64 states: 509 us
+// with four, 454 with one; 30 of 140 + 126 FP32 states: 377 with two, 338 with one).
 GainPass gain_pass(int elem_size, int f_smem_len, int max_n2p, int n_cells) {
     GainPass p;
-    const int nvr = max_n2p * elem_size / 16;
+    const int nvr = max_n2p * elem_size / 16, n = 16 / elem_size;
     p.kv = nvr <= kGainConsumers ? 1 : (nvr <= 2 * kGainConsumers ? 2 : 4);
     if (elem_size == 8 && n_cells > 2) p.kv = std::max(p.kv, 2);
-    int most = std::min(kGainMaxCells, 32 / (p.kv * (16 / elem_size)));
-    while (most > 1 && gain_stream_smem_bytes(elem_size, f_smem_len, most) > kGainSmemLimit) --most;
+    if (elem_size == 4 && n_cells == 1 && nvr >= 4 * 32) p.kv = 4;
+    int most = std::min(kGainMaxCells, 32 / (p.kv * n));
     if (elem_size == 8 && p.kv == 1) most = std::min(most, 2);
+    while (most > 1 && gain_stream_smem_bytes(elem_size, f_smem_len, most) > kGainSmemLimit) --most;
     const int passes = (n_cells + most - 1) / most;
     p.cells = passes > 0 ? (n_cells + passes - 1) / passes : 1;
     return p;
@@ -531,118 +315,48 @@ __global__ void __launch_bounds__(kRowsWarps * 32) euler_rows_kernel(RowOps<T> o
     double s_df = 0.0, s_f = 0.0;
     const int cell = i < ops.n_state ? i / ops.n_mom : 0;
     const int a = i - cell * ops.n_mom;
-    const T* fc = f_in + (size_t)cell * ops.n_mom;
     int s = 0;
-    double flux = 0.0, emi = 0.0, loss = 0.0, gain = 0.0;
+    double flux = 0.0, emi = 0.0, loss = 0.0;
     // binary term of this cell (SteppingMethods.jl:369): outside BinM.Domain it is zero
     const bool bin_here = i < ops.n_state && ops.has_bin && (ops.bin_on == nullptr || ops.bin_on[cell] != 0);
-    if (i < ops.n_state) {
-        while (s + 1 < ops.n_species && a >= ops.sp_off[s + 1]) ++s;
-
-        // (a) banded flux row: ELL slots of width ell_w, 128-bit loads of 4 slots per lane
-        {
-            const T* vrow = ops.ell_val + (size_t)i * ops.ell_w;
-            const int* crow = ops.ell_col + (size_t)i * ops.ell_w;
-            for (int k = lane * 4; k < ops.ell_w; k += 128) {
-                const int4 c4 = *reinterpret_cast<const int4*>(crow + k);
-                T v0, v1, v2, v3;
-                if constexpr (sizeof(T) == 4) {
-                    const float4 v4 = *reinterpret_cast<const float4*>(vrow + k);
-                    v0 = v4.x; v1 = v4.y; v2 = v4.z; v3 = v4.w;
-                } else {
-                    const double2 va = *reinterpret_cast<const double2*>(vrow + k);
-                    const double2 vb = *reinterpret_cast<const double2*>(vrow + k + 2);
-                    v0 = va.x; v1 = va.y; v2 = vb.x; v3 = vb.y;
-                }
-                // padding slots carry column -1: only stored entries take part, like a CSC product
-                if (c4.x >= 0) flux += (double)v0 * (double)f_in[c4.x];
-                if (c4.y >= 0) flux += (double)v1 * (double)f_in[c4.y];
-                if (c4.z >= 0) flux += (double)v2 * (double)f_in[c4.z];
-                if (c4.w >= 0) flux += (double)v3 * (double)f_in[c4.w];
-            }
-        }
-        // (c) emission row pieces
-        if (ops.has_emi) {
-            for (int p = ops.emi_rptr[i]; p < ops.emi_rptr[i + 1]; ++p) {
-                const int pc = ops.emi_piece[p];
-                const T* row = ops.emi_data + ops.emi_data_off[pc] + (size_t)(i - ops.emi_row0[pc]) * ops.emi_ld[pc];
-                const T* fx = f_in + ops.emi_col0[pc];
-                const int nc = ops.emi_ncols[pc];
-                for (int c = lane; c < nc; c += 32) emi += (double)row[c] * (double)fx[c];
-            }
-        }
-        // loss bilinear term
-        if (bin_here) {
-            const int la = a - ops.sp_off[s];
-            for (int b = ops.loss_ptr[s]; b < ops.loss_ptr[s + 1]; ++b) {
-                const T* row = ops.loss_data + ops.loss_data_off[b] + (size_t)la * ops.loss_ld[b];
-                const T* fx = fc + ops.loss_col_off[b];
-                const int nc = ops.loss_ncols[b];
-                for (int c = lane; c < nc; c += 32) loss += (double)row[c] * (double)fx[c];
-            }
-        }
-        flux = warp_sum(flux);
-        emi = warp_sum(emi);
-        loss = warp_sum(loss);
-    }
     // The row's unit range, old state and vectors are static or the previous step's: read them
     // before the wait too, so only the gain partials' round trip follows it.
     int u_lo = 0, u_hi = 0;
     T fa = T(0), iap = T(0), injv = T(0), volc = T(0);
     if (i < ops.n_state) {
+        while (s + 1 < ops.n_species && a >= ops.sp_off[s + 1]) ++s;
+        row_terms(ops, i, cell, a, s, bin_here, lane, [f_in](int k) { return (double)f_in[k]; }, flux, emi, loss);
         if (bin_here) {
             u_lo = ops.unit_ptr[a];
             u_hi = ops.unit_ptr[a + 1];
+            volc = ops.vol[cell];
         }
-        if (lane == 0) {
-            fa = fc[a];
-            iap = ops.invAp[i];
-            if (ops.mode == 0) injv = ops.inj[i];
-            if (bin_here) volc = ops.vol[cell];
-        }
+        fa = f_in[i];
+        iap = ops.invAp[i];
+        if (ops.mode == 0) injv = ops.inj[i];
     }
     pdl_wait();  // this step's gain partials (and, in the space pass, the momentum pass) are complete
     if (threadIdx.x == 0) pdl_trigger();
     if (i < ops.n_state) {
-        if (bin_here) {
-            const double* pr = ops.partial + (size_t)cell * ops.n_units;
-            for (int u = u_lo + lane; u < u_hi; u += 32) gain += pr[u];
-        }
-        gain = warp_sum(gain);
-
+        const double* pr = ops.partial + (size_t)cell * ops.n_units;
+        const double gain = sum_partials(pr, u_lo, u_hi);
+        T dbin;
+        const T df = row_df(ops, bin_here, fa, iap, volc, flux, emi, loss, gain, dt_scale, dbin);
         if (lane == 0 && ops.mode == 1) {
             // ForwardSymplecticEuler momentum pass (SteppingMethods.jl:140-160)
-            T df = -(T)flux;
-            if (ops.has_emi) df = df + (T)emi;
-            if (ops.has_bin) df = df + (bin_here ? (T)((double)volc * (gain - (double)fa * loss)) : T(0));
-            df = (T)((double)df * ((double)iap * dt_scale));
-            T fm = fa + df;
-            fm = jl_mul_bool(fm, fm >= (T)ops.thr_mom);
-            f_out[i] = fm;
+            const T fm = fa + df;
+            f_out[i] = jl_mul_bool(fm, fm >= (T)ops.thr_mom);
             ops.dfm_out[i] = df;
         }
         if (lane == 0 && ops.mode == 0) {
-            const T dflux = (T)flux;
-            const T demi = (T)emi;
-            const T dbin = bin_here ? (T)((double)volc * (gain - (double)fa * loss)) : T(0);
-            // SteppingMethods.jl:31-46
-            T df = -dflux;
-            if (ops.has_emi) df = df + demi;
-            if (ops.has_bin) df = df + dbin;
-            df = (T)((double)df * ((double)iap * dt_scale));
-            // :97-101, arithmetic in Float64 like Julia's promotion, one rounding at the store
-            const double fnew = (double)fa + ((double)df + (double)injv * dt_scale);
-            T fn = (T)fnew;
-            fn = jl_mul_bool(fn, fn >= (T)ops.thr);
-            fn = jl_mul_bool(fn, fn != (T)CUDART_INF);
-            f_out[i] = fn;
+            f_out[i] = row_update(ops, fa, df, injv, dt_scale);
             // :48-94 diagnostics on the old f
             const double fd = (double)fa;
             m_cr = nan_to_inf((double)df / fd);
             if (verbose == 3) {
                 if (ops.has_bin) m_bin = nan_to_inf((double)dbin / fd);
-                if (ops.has_emi) m_emi = nan_to_inf((double)demi / fd);
-                m_flux = nan_to_inf(-(double)dflux / fd);
+                if (ops.has_emi) m_emi = nan_to_inf((double)(T)emi / fd);
+                m_flux = nan_to_inf(-(double)(T)flux / fd);
             }
             s_df = (double)df;
             s_f = fd;
@@ -661,10 +375,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32) euler_rows_kernel(RowOps<T> o
     }
     __syncthreads();
     if (threadIdx.x < kStepRecFields) {
-        // one thread per field, the warps in order: fields 0-3 are minima, 4-5 sums
-        const int k = threadIdx.x;
+        const int k = threadIdx.x;  // one thread per field, the warps in order
         double r = s_red[0][k];
-        for (int w = 1; w < kRowsWarps; ++w) r = k < 4 ? jl_min(r, s_red[w][k]) : r + s_red[w][k];
+        for (int w = 1; w < kRowsWarps; ++w) r = rec_join(k, r, s_red[w][k]);
         rec[(size_t)blockIdx.x * kStepRecFields + k] = r;
     }
 }
@@ -689,10 +402,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) step_diag_kernel(const double
     const double* recs = blk_red + (size_t)blockIdx.x * n_blocks * kStepRecFields;
     double r[kStepRecFields] = {CUDART_INF, CUDART_INF, CUDART_INF, CUDART_INF, 0.0, 0.0};
     for (int b = threadIdx.x; b < n_blocks; b += blockDim.x) {
-        const double* src = recs + (size_t)b * kStepRecFields;
-        for (int k = 0; k < 4; ++k) r[k] = jl_min(r[k], __ldcg(src + k));
-        r[4] += __ldcg(src + 4);
-        r[5] += __ldcg(src + 5);
+        for (int k = 0; k < kStepRecFields; ++k) r[k] = rec_join(k, r[k], __ldcg(recs + (size_t)b * kStepRecFields + k));
     }
     for (int k = 0; k < kStepRecFields; ++k) s_fin[k][threadIdx.x] = r[k];
     __syncthreads();
@@ -777,18 +487,12 @@ __global__ void __launch_bounds__(kRowsWarps * 32) sympl_space_kernel(RowOps<T> 
         double xf = 0.0;
         for (int k = lane; k < ops.x_ell_w; k += 32) {
             const int c = ops.x_ell_col[(size_t)i * ops.x_ell_w + k];
-            if (c >= 0) xf += (double)ops.x_ell_val[(size_t)i * ops.x_ell_w + k] * (double)fm[c];
+            if (c >= 0) xf = fma((double)ops.x_ell_val[(size_t)i * ops.x_ell_w + k], (double)fm[c], xf);
         }
         xf = warp_sum(xf);
         if (lane == 0) {
-            const T dsp = (T)((double)(-(T)xf * ops.invAp[i]) * dt_scale);
-            T fs = fm[i] + dsp;
-            fs = jl_mul_bool(fs, fs >= (T)ops.thr_space);
-            T v = (T)((double)fs + (double)ops.inj[i] * dt_scale);
-            const T sg = isnan(v) ? v : (v > T(0) ? T(1) : (v < T(0) ? T(-1) : v));
-            v = jl_mul_bool(v, v >= (T)ops.thr_space) * sg;
-            v = jl_mul_bool(v, v != (T)CUDART_INF);
-            f_out[i] = v;
+            T dsp;
+            f_out[i] = row_space_update(ops, fm[i], xf, ops.invAp[i], ops.inj[i], dt_scale, dsp);
             const double fo = (double)f_old[i];
             m_cr = nan_to_inf((double)(dsp + dfm[i]) / fo);
             s_f = fo;
