@@ -140,6 +140,11 @@ struct dtb_ctx {
     int n_units = 0;
     int gain_grid = 0;
     GainPass gain_pass;
+    // many steps per launch with the units in shared memory (kernels_resident.cu)
+    bool res_on = false;
+    GainPass res_pass;
+    ResidentArgs res{};
+    int res_grid = 0, res_smem = 0;
     int f_smem_len = 0;
     int* unit_ptr = nullptr;
     double* partial = nullptr;

@@ -549,6 +549,50 @@ static void sparse_runs(const SparseGain& g, int64_t n2p, int64_t max_elems, std
     if (!rows.empty()) flush(r0, rows.size(), u0, u1);
 }
 
+// Whether runs may use the kernel that keeps the gain units in shared memory: the library's choice
+// of how to run steps (opts.graph_steps 0), every cell in the binary domain, and a state that one
+// block can update.
+static bool resident_eligible(const dtb_ctx* c) {
+    int coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
+    return coop && c->opts.graph_steps == 0 && c->n_bin_cells == c->n_space && !c->has_bin_domain &&
+           c->n_state <= resident_max_states();
+}
+
+// Device arrays of that kernel, once the flux is known.
+template <typename T>
+static int commit_resident(dtb_ctx* c, const RowOps<T>& ops, const std::vector<int>& first,
+                           const std::vector<int>& own, const std::vector<int>& slot) {
+    if (!c->res_on) return DTB_OK;
+    int bps = 0;
+    const bool fits = (!c->symplectic || ops.x_ell_w <= kResMaxX) &&
+                      prepare_resident<T>(c->res_pass, c->symplectic, (int)c->n_state, c->res_smem, &bps) == cudaSuccess && bps >= 1;
+    if (!fits) {
+        cudaGetLastError();
+        c->res_on = false;
+        return DTB_OK;
+    }
+    ResidentArgs& r = c->res;
+    int *d_first, *d_own, *d_slot;
+    DTB_TRY(copy_host_ints(c, &d_first, first));
+    DTB_TRY(copy_host_ints(c, &d_own, own));
+    DTB_TRY(copy_host_ints(c, &d_slot, slot));
+    const size_t part_bytes = 16 * 2 * (kResSegs - 1) * (size_t)c->n_state, next_bytes = 16 * 2 * (size_t)c->n_state;
+    DTB_TRY(c->alloc(&r.partial, part_bytes));
+    DTB_TRY(c->alloc(&r.next, next_bytes));
+    DTB_TRY(c->alloc(&r.diag, sizeof(double) * kStepRecFields * (size_t)c->graph_steps * c->n_state));
+    DTB_CUDA(cudaMemsetAsync(r.partial, 0, part_bytes, c->stream));  // no word carries a step's number yet
+    DTB_CUDA(cudaMemsetAsync(r.next, 0, next_bytes, c->stream));
+    r.base = 0;
+    r.G = c->G_all;
+    r.units = c->units;
+    r.first = d_first;
+    r.own = d_own;
+    r.slot = d_slot;
+    r.f_len = c->f_smem_len;
+    return DTB_OK;
+}
+
 template <typename T>
 static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
     const size_t esz = sizeof(T);
@@ -700,6 +744,7 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
     std::vector<GainUnit> units;
     std::vector<int> unit_ptr((size_t)c->n_mom + 1, 0);
     int unit_row = 0;
+    std::vector<int> res_first, res_own, res_slot;
     {
         double tot_bytes = sparse_bytes;
         for (auto& b : blks) tot_bytes += (double)b.no * b.n1 * b.n2 * esz;
@@ -769,6 +814,72 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
                 target = t;
             }
         }
+        // A grid whose units fit the SMs' shared memory is planned for the kernel that keeps them
+        // there: the units in order, cut into one run of nearly equal bytes per SM, judged by the
+        // fullest group of threads of a block.
+        if (resident_eligible(c)) {
+            c->res_pass = resident_pass((int)esz, c->gain_pass, c->n_space);
+            const bool pad = c->offp[c->ns] != c->n_mom;
+            double res_best = 0;
+            for (double t = 256.0 * 1024; t >= kGainTileBytes; t -= t > 128.0 * 1024 ? 32768 : 16384) {
+                std::vector<std::pair<int, int64_t>> list;  // (row, bytes) of every unit
+                each_unit(t, [&](const GainUnit& w) { list.push_back({w.row, (int64_t)w.nb * w.n2p * (int64_t)esz}); });
+                const size_t n = list.size(), grid = std::min<size_t>(n, (size_t)c->num_sms);
+                if (n == 0 || n > grid * 256) break;
+                const double cost = 4096;  // what a unit costs beside its bytes
+                double total = 0, cum = 0;
+                for (auto& w : list) total += (double)w.second + cost;
+                std::vector<int> first(grid + 1, (int)n), own(grid + 1, (int)c->n_mom), slot(n, 0);
+                std::vector<int64_t> bytes(grid, 0);
+                double group = 0;
+                int max_local = 0, max_own = 0, segs = 0, row = 0;
+                size_t u = 0;
+                for (size_t blk = 0; blk < grid; ++blk) {
+                    first[blk] = (int)u;
+                    const double upto = total * (double)(blk + 1) / (double)grid;
+                    double part[kResGroups] = {};
+                    // at least one unit each, and one left for every block to come
+                    while (u < n - (grid - 1 - blk) &&
+                           (u == (size_t)first[blk] || cum + 0.5 * ((double)list[u].second + cost) <= upto ||
+                            blk + 1 == grid)) {
+                        cum += (double)list[u].second + cost;
+                        bytes[blk] += list[u].second;
+                        part[(u - (size_t)first[blk]) % kResGroups] += (double)list[u].second + cost;
+                        if (u > 0 && list[u].first == list[u - 1].first)
+                            slot[u] = slot[u - 1] + (u == (size_t)first[blk] ? 1 : 0);
+                        segs = std::max(segs, slot[u] + 1);
+                        ++u;
+                    }
+                    max_local = std::max(max_local, (int)u - first[blk]);
+                    for (double p : part) group = std::max(group, p);
+                    // the rows whose units start here (and those without units up to the next that do)
+                    own[blk] = blk == 0 ? 0 : row;
+                    row = u < n ? (slot[u - 1] >= 0 && list[u].first == list[u - 1].first ? list[u].first + 1 : list[u].first)
+                                : (int)c->n_mom;
+                    if (blk > 0) max_own = std::max(max_own, own[blk] - own[blk - 1]);
+                    if (blk + 1 == grid) max_own = std::max(max_own, (int)c->n_mom - own[blk]);
+                }
+                const int64_t g = *std::max_element(bytes.begin(), bytes.end());
+                if (u != n || segs > kResSegs || g > kGainSmemLimit || c->n_mom > 65535) continue;
+                const int smem = resident_smem_bytes(c->res_pass, (int)esz, (int)g, (int)c->offp[c->ns], c->n_space,
+                                                     (int)c->n_state, pad, max_local, max_own);
+                if (smem > kGainSmemLimit) continue;
+                if (!c->res_on || group < res_best) {
+                    res_best = group;
+                    target = t;
+                    c->res_on = true;
+                    c->res_grid = (int)grid;
+                    c->res_smem = smem;
+                    c->res.g_bytes = (int)g;
+                    c->res.max_local = max_local;
+                    c->res.max_own = max_own;
+                    c->res.pad = pad;
+                    res_first.swap(first);
+                    res_own.swap(own);
+                    res_slot.swap(slot);
+                }
+            }
+        }
         each_unit(target, [&](const GainUnit& u) {
             while (unit_row < u.row) unit_ptr[(size_t)++unit_row] = (int)units.size();
             units.push_back(u);
@@ -779,6 +890,20 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
     c->gain_grid = std::max(1, std::min(c->n_units, c->num_sms * bps));
     DTB_TRY(copy_host_ints(c, &c->units, units));
     DTB_TRY(copy_host_ints(c, &c->unit_ptr, unit_ptr));
+    {
+        // the rows' segments: cut where the units pass from one block's shared memory to the next's
+        std::vector<int2> cuts((size_t)c->n_mom);
+        for (int64_t a = 0; a < c->n_mom; ++a) {
+            const int lo = unit_ptr[(size_t)a], hi = unit_ptr[(size_t)a + 1];
+            int2 cut = make_int2(hi, hi);
+            for (int u = hi - 1; u > lo && c->res_on; --u)
+                if (res_slot[(size_t)u] != res_slot[(size_t)u - 1]) (res_slot[(size_t)u] == 1 ? cut.x : cut.y) = u;
+            cuts[(size_t)a] = cut;
+        }
+        int2* d_cuts;
+        DTB_TRY(copy_host_ints(c, &d_cuts, cuts));
+        ops.cuts = d_cuts;
+    }
     DTB_TRY(c->alloc(&c->partial, sizeof(double) * (size_t)std::max(1, c->n_units) * c->n_space));
     DTB_CUDA(cudaMemsetAsync(c->partial, 0, sizeof(double) * (size_t)std::max(1, c->n_units) * c->n_space,
                              c->stream));
@@ -918,7 +1043,7 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
     ops.thr = c->prec == DTB_F64 ? (double)1e-10f : (double)(T)1e-10f;
     ops.has_bin = c->has_bin;
     ops.has_emi = c->has_emi;
-    return DTB_OK;
+    return commit_resident<T>(c, ops, res_first, res_own, res_slot);
 }
 
 extern "C" int32_t dtb_commit(dtb_ctx* c) {
@@ -1048,12 +1173,12 @@ static int do_step(dtb_ctx* c, double dt_imm, bool use_arr, int verbose, bool pr
 }
 
 // The diagnostics of the last n steps (a sequence of record slots 0..n-1) and the counter advance.
-static int finish_seq(dtb_ctx* c, int n, int verbose) {
+static int finish_seq(dtb_ctx* c, int n, int verbose, bool resident = false) {
     if (n <= 0) return DTB_OK;
     const int hb = c->prec == DTB_F64 ? c->ops_d.has_bin : c->ops_f.has_bin;
     const int he = c->prec == DTB_F64 ? c->ops_d.has_emi : c->ops_f.has_emi;
-    DTB_CUDA(launch_step_diag(c->blk_red, c->rows_grid, n, c->ctr, c->hist, c->hist_cap, verbose, hb, he,
-                              c->symplectic ? 1 : 0, c->ticket, c->stream));
+    DTB_CUDA(launch_step_diag(resident ? c->res.diag : c->blk_red, c->rows_grid, n, c->ctr, c->hist, c->hist_cap, verbose,
+                              hb, he, c->symplectic ? 1 : 0, c->ticket, resident ? (int)c->n_state : 0, c->stream));
     c->launches++;
     return DTB_OK;
 }
@@ -1067,6 +1192,30 @@ static int run_loose(dtb_ctx* c, int64_t n, int verbose, bool profile) {
         done += m;
     }
     return DTB_OK;
+}
+
+// n steps of the resident kernel, a launch per sequence of at most graph_steps (the record slots).
+template <typename T>
+static int run_resident_typed(dtb_ctx* c, const RowOps<T>& ops, int64_t n, int verbose) {
+    c->res.err = c->err;
+    for (int64_t done = 0; done < n;) {
+        const int m = (int)std::min<int64_t>(c->graph_steps, n - done);
+        DTB_CUDA(launch_resident<T>(c->res_pass, ops, c->res, c->sp_off_host,
+                                    reinterpret_cast<const T*>(c->f_buf[c->cur]),
+                                    reinterpret_cast<T*>(c->f_buf[c->cur ^ 1]), c->dt_arr, c->ctr, m, verbose, c->res_grid,
+                                    c->res_smem, c->symplectic, c->stream));
+        c->res.base += (unsigned long long)m;
+        c->launches++;
+        c->cur ^= 1;
+        c->host_ctr += m;
+        DTB_TRY(finish_seq(c, m, verbose, true));
+        done += m;
+    }
+    return DTB_OK;
+}
+static int run_resident(dtb_ctx* c, int64_t n, int verbose) {
+    return c->prec == DTB_F64 ? run_resident_typed<double>(c, c->ops_d, n, verbose)
+                              : run_resident_typed<float>(c, c->ops_f, n, verbose);
 }
 
 static int check_kernel_err(dtb_ctx* c) {
@@ -1120,6 +1269,7 @@ static int run_chunk(dtb_ctx* c, int64_t n, int verbose, bool use_graph) {
     DTB_CUDA(cudaMemsetAsync(c->ctr, 0, sizeof(unsigned long long), c->stream));
     c->host_ctr = 0;
     int64_t done = 0;
+    if (use_graph && c->res_on && !c->profiling && n >= c->graph_steps) return run_resident(c, n, verbose);
     if (use_graph && !c->profiling && n >= c->graph_steps) {
         if (c->cur != 0) {
             DTB_TRY(run_loose(c, 1, verbose, false));
@@ -1237,7 +1387,7 @@ int32_t dtb_prepare(dtb_ctx* c) {
     DTB_TRY(dtb_commit(c));
     DeviceGuard g(c->device);
     if (c->prec == DTB_MIXED) return batch_prepare(c);
-    if (c->profiling) return DTB_OK;  // profiled runs launch step by step
+    if (c->profiling || c->res_on) return DTB_OK;  // profiled runs launch step by step; no graph to capture
     DTB_TRY(ensure_graph(c, 0));
     DTB_CUDA(cudaGraphUpload(c->graph, c->stream));
     DTB_CUDA(cudaStreamSynchronize(c->stream));
@@ -1377,10 +1527,15 @@ static int ensure_pipe(dtb_ctx* c) {
     return DTB_OK;
 }
 
-// n steps through the device counter from its current value (graph replays where they fit).
+// Save intervals of this many steps and more pay for loading the units into shared memory.
+constexpr int64_t kResMinSteps = 8;
+
+// n steps through the device counter from its current value (the resident kernel or graph replays
+// where they fit).
 static int run_steps(dtb_ctx* c, int64_t n, int verbose) {
     int64_t done = 0;
-    if (!c->profiling && n >= c->graph_steps) {
+    if (c->res_on && !c->profiling && n >= kResMinSteps) return run_resident(c, n, verbose);
+    if (!c->res_on && !c->profiling && n >= c->graph_steps) {
         if (c->cur != 0) {
             DTB_TRY(run_loose(c, 1, verbose, false));
             done++;
@@ -1415,7 +1570,7 @@ extern "C" int32_t dtb_solve_ex(dtb_ctx* c, double dt_initial, const double* t_s
     const bool want_diag = verbose == 1 || verbose == 2 || verbose == 3;
     if (want_diag && !c->pin_hist2)
         DTB_CUDA(cudaMallocHost(&c->pin_hist2, sizeof(StepDiagDev) * 2 * (size_t)c->hist_cap));
-    if (!c->profiling) DTB_TRY(ensure_graph(c, verbose));
+    if (!c->profiling && !c->res_on) DTB_TRY(ensure_graph(c, verbose));
     const size_t fb = c->esz * (size_t)c->n_state;
     const size_t mstride = (size_t)2 * c->ns * c->n_space;
     double* mom_all = nullptr;

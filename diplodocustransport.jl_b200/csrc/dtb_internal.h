@@ -74,6 +74,10 @@ struct RowOps {
     const T* loss_data;
     // gain partials: units of row a are [unit_ptr[a], unit_ptr[a+1])
     const int* unit_ptr;
+    // a row's units fall into at most three segments, [unit_ptr[a], cuts[a].x), [cuts[a].x, cuts[a].y)
+    // and the rest: its gain is the sum of the segments' sums (one segment unless the units of the
+    // row live in the shared memory of several blocks, see launch_resident)
+    const int2* cuts;
     int n_units;
     const double* partial;                 // [n_space][n_units]
     const unsigned char* bin_on;           // per cell: binary term applied (BinM.Domain); null = all
@@ -127,10 +131,46 @@ int euler_rows_blocks(int n_state);
 // The diagnostics of steps *ctr .. *ctr + n_steps - 1: block k reduces step k's row-block
 // records (slot k of blk_red, n_blocks records of kStepRecFields each) into
 // hist[(*ctr + k) % hist_cap]; the last block to finish advances *ctr by n_steps. sympl: the
-// records are the symplectic space pass's (no per-term Crs, no finite check).
+// records are the symplectic space pass's (no per-term Crs, no finite check). n_state > 0: blk_red
+// holds the resident kernel's terms per state (ResidentArgs::diag), divided and joined eight by eight
+// first, as euler_rows does.
 cudaError_t launch_step_diag(const double* blk_red, int n_blocks, int n_steps, unsigned long long* ctr,
                              StepDiagDev* hist, long long hist_cap, int verbose, int has_bin, int has_emi, int sympl,
-                             unsigned* ticket, cudaStream_t s);
+                             unsigned* ticket, int n_state, cudaStream_t s);
+
+// Many steps in one cooperative launch with the work units in shared memory
+// (kernels_resident.cu). Block b holds units [first[b], first[b + 1]) and owns rows
+// [own[b], own[b + 1]); a row's units in one block are a segment (slot 0 in its owner).
+// partial: two buffers of [kResSegs - 1][n_state] 16-byte words; next: two of [n_state]; base: steps
+// of the launches before (the words' step numbers go on from there).
+constexpr int kResMaxX = 8;    // slots of the X flux's rows
+constexpr int kResGroups = 2;  // groups of threads that take a work unit each at a time
+constexpr int kResSegs = 3;    // segments of a row
+struct ResidentArgs {
+    const void* G;
+    const GainUnit* units;
+    const int* first;  // [blocks + 1]
+    const int* own;    // [blocks + 1]
+    const int* slot;   // per unit: the segment of its row
+    int max_local, max_own;  // units and owned rows of the fullest block
+    int g_bytes, f_len, pad;
+    void* partial;
+    void* next;
+    double* diag;      // per step and state: df, its parts by M_Bin, emission and flux (verbose 3), -, old f,
+                       // [steps][kStepRecFields][n_state]
+    unsigned long long base;
+    int* err;
+};
+int resident_smem_bytes(const GainPass& p, int elem_size, int g_bytes, int f_len, int n_space, int n_state, bool pad,
+                        int max_local, int max_own);
+GainPass resident_pass(int elem_size, const GainPass& g, int n_space);
+int resident_max_states();
+template <typename T>
+cudaError_t prepare_resident(const GainPass& p, bool sy, int n_state, int smem, int* blocks_per_sm);
+template <typename T>
+cudaError_t launch_resident(const GainPass& p, const RowOps<T>& ops, const ResidentArgs& r, const int* sp_off_host,
+                            const T* f_in, T* f_out, const double* dt_arr, const unsigned long long* ctr, int n_steps,
+                            int verbose, int grid, int smem, bool sy, cudaStream_t s);
 
 // The symplectic space pass of a step numbered like launch_euler_rows'; its row blocks write
 // records in the same layout (the whole-step Cr and the f sum only).

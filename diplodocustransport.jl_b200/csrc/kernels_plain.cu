@@ -322,6 +322,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) euler_rows_kernel(RowOps<T> o
     // The row's unit range, old state and vectors are static or the previous step's: read them
     // before the wait too, so only the gain partials' round trip follows it.
     int u_lo = 0, u_hi = 0;
+    int2 cut = make_int2(0, 0);
     T fa = T(0), iap = T(0), injv = T(0), volc = T(0);
     if (i < ops.n_state) {
         while (s + 1 < ops.n_species && a >= ops.sp_off[s + 1]) ++s;
@@ -329,6 +330,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) euler_rows_kernel(RowOps<T> o
         if (bin_here) {
             u_lo = ops.unit_ptr[a];
             u_hi = ops.unit_ptr[a + 1];
+            cut = ops.cuts[a];
             volc = ops.vol[cell];
         }
         fa = f_in[i];
@@ -339,7 +341,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) euler_rows_kernel(RowOps<T> o
     if (threadIdx.x == 0) pdl_trigger();
     if (i < ops.n_state) {
         const double* pr = ops.partial + (size_t)cell * ops.n_units;
-        const double gain = sum_partials(pr, u_lo, u_hi);
+        const double gain = sum_partials(pr, u_lo, cut, u_hi);
         T dbin;
         const T df = row_df(ops, bin_here, fa, iap, volc, flux, emi, loss, gain, dt_scale, dbin);
         if (lane == 0 && ops.mode == 1) {
@@ -392,17 +394,33 @@ __global__ void __launch_bounds__(kRowsWarps * 32) step_diag_kernel(const double
                                                                     unsigned long long* ctr, StepDiagDev* hist,
                                                                     long long hist_cap, int verbose,
                                                                     int has_bin, int has_emi, int sympl,
-                                                                    unsigned* ticket) {
+                                                                    unsigned* ticket, int n_state) {
     __shared__ double s_fin[kStepRecFields][kRowsWarps * 32];
     pdl_wait();  // the last step's row blocks have written their records
     // a gain kernel that follows may start streaming its (static) blocks; it reads the state and
     // the row kernel after it reads the counter only after this grid has finished
     if (threadIdx.x == 0) pdl_trigger();
     const unsigned long long step0 = *reinterpret_cast<volatile unsigned long long*>(ctr);
-    const double* recs = blk_red + (size_t)blockIdx.x * n_blocks * kStepRecFields;
+    const double* recs = blk_red + (size_t)blockIdx.x * (n_state > 0 ? n_state : n_blocks) * kStepRecFields;
     double r[kStepRecFields] = {CUDART_INF, CUDART_INF, CUDART_INF, CUDART_INF, 0.0, 0.0};
     for (int b = threadIdx.x; b < n_blocks; b += blockDim.x) {
-        for (int k = 0; k < kStepRecFields; ++k) r[k] = rec_join(k, r[k], __ldcg(recs + (size_t)b * kStepRecFields + k));
+        for (int k = 0; k < kStepRecFields; ++k) {
+            double v;
+            if (n_state > 0) {  // the record's rows in order, as euler_rows joins them
+                const bool in = k == 0 || (k == 1 ? has_bin != 0 : k == 2 ? has_emi != 0 : true);
+                if (k >= 1 && k <= 3 && (verbose != 3 || sympl)) continue;
+                const auto field = [&](int i) {
+                    const double fd = __ldcg(recs + 5 * (size_t)n_state + i);
+                    if (k >= 4) return k == 5 ? fd : (sympl ? 0.0 : __ldcg(recs + i));
+                    return in ? nan_to_inf(__ldcg(recs + (size_t)k * n_state + i) / fd) : CUDART_INF;
+                };
+                v = field(b * kRowsWarps);
+                for (int i = b * kRowsWarps + 1; i < min(n_state, (b + 1) * kRowsWarps); ++i) v = rec_join(k, v, field(i));
+            } else {
+                v = __ldcg(recs + (size_t)b * kStepRecFields + k);
+            }
+            r[k] = rec_join(k, r[k], v);
+        }
     }
     for (int k = 0; k < kStepRecFields; ++k) s_fin[k][threadIdx.x] = r[k];
     __syncthreads();
@@ -440,9 +458,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32) step_diag_kernel(const double
 
 cudaError_t launch_step_diag(const double* blk_red, int n_blocks, int n_steps, unsigned long long* ctr,
                              StepDiagDev* hist, long long hist_cap, int verbose, int has_bin, int has_emi, int sympl,
-                             unsigned* ticket, cudaStream_t s) {
+                             unsigned* ticket, int n_state, cudaStream_t s) {
     return launch_pdl(step_diag_kernel, dim3(n_steps), dim3(kRowsWarps * 32), 0, s, blk_red, n_blocks, n_steps, ctr,
-                      hist, hist_cap, verbose, has_bin, has_emi, sympl, ticket);
+                      hist, hist_cap, verbose, has_bin, has_emi, sympl, ticket, n_state);
 }
 
 template <typename T>

@@ -1,5 +1,6 @@
-// Device pieces of the plain Euler step (kernels_plain.cu): barriers and bulk copies, a work unit's
-// contraction, and a row's terms and update.
+// Device pieces of the plain Euler step shared by the streaming kernels (kernels_plain.cu) and the
+// resident one (kernels_resident.cu): barriers and bulk copies, a work unit's contraction and a
+// row's terms and update. Both run them on the same work table, so their steps agree bit for bit.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -287,6 +288,7 @@ __device__ __forceinline__ void stage_f(typename StagedT<T, C>::type* f_s, const
 }
 
 // ------------------------------------------------------------------ one row of the step
+// The pieces of a row's step, shared by the kernels that run it so that they agree bit for bit.
 
 // Flux, emission and loss sums of state row i (row a of species s in its cell) over one warp.
 // f_at(k): the step's input state k in FP64.
@@ -345,18 +347,25 @@ __device__ __forceinline__ void row_terms(const RowOps<T>& ops, int i, int cell,
     loss = __shfl_sync(0xffffffffu, sum, 16);
 }
 
-// Gain partials lo .. hi - 1 in unit order, eight loads in flight (from L2: other blocks wrote them).
-__device__ __forceinline__ double sum_partials(const double* pr, int lo, int hi) {
-    double gain = 0.0;
+// A row's gain: the sums of its (at most three) segments of units, in order (RowOps::cuts).
+__device__ __forceinline__ double row_gain(double a, double b, double c) { return a + b + c; }
+
+// The gain from partials lo .. hi - 1, in unit order within the segments, eight loads in flight
+// (from L2: other blocks wrote them).
+__device__ __forceinline__ double sum_partials(const double* pr, int lo, int2 cut, int hi) {
+    double a = 0.0, b = 0.0, c = 0.0;
     for (int u = lo; u < hi; u += 8) {
         double v[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = u + k < hi ? __ldcg(pr + u + k) : 0.0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (u + k < hi) gain += v[k];
+        for (int k = 0; k < 8; ++k) {
+            if (u + k < min(cut.x, hi)) a += v[k];
+            else if (u + k < min(cut.y, hi)) b += v[k];
+            else if (u + k < hi) c += v[k];
+        }
     }
-    return gain;
+    return row_gain(a, b, c);
 }
 
 // df of a row before and after its scaling (SteppingMethods.jl:31-46).
