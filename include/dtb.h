@@ -71,7 +71,11 @@ typedef struct dtb_opts {
     int32_t index_base;    /* base of sparse indices the caller passes: 1 (Julia) or 0 */
     int32_t graph_steps;   /* steps per captured CUDA graph (at most 1024). 0: the default, for
                               plain contexts 64 when the step records of 64 steps fit in 8 MB
-                              (grids up to about 175,000 states) and 16 above; 16 for batched ones */
+                              (grids up to about 175,000 states) and 16 above; 16 for batched
+                              ones. 0 also lets longer runs of a plain context on a small grid
+                              (gain blocks up to about 33 MB) keep the gain in shared memory, one
+                              launch for 64 steps, with the same results bit for bit; any other
+                              value keeps two launches per step */
     double dt0;            /* TimeStruct.dt0 (StructsAndDictionaries.jl:55) */
     int32_t batch;         /* instances per context; 1 for the plain method */
     int32_t flags;         /* reserved, 0 */
@@ -179,8 +183,9 @@ int32_t dtb_step_io(dtb_ctx* ctx, const double* f_in, double* f_out, double t_st
 /* Captures, instantiates and uploads the CUDA graphs that dtb_run (Verbose = 0) or, for a
  * batched context, dtb_batch_run replay, without running a step (commits first if needed).
  * Optional: without it the first run long enough for a graph captures it. A caller that times
- * its steps calls it once beforehand so no capture falls inside the timed steps. No
- * counterpart in the reference (its Julia loop has no graphs). */
+ * its steps calls it once beforehand so no capture falls inside the timed steps. A context whose
+ * runs keep the gain in shared memory (opts.graph_steps) has no graphs to capture. No counterpart
+ * in the reference (its Julia loop has no graphs). */
 int32_t dtb_prepare(dtb_ctx* ctx);
 
 /* nsteps steps with the given dt/dt0 values, replayed from captured CUDA graphs.
@@ -227,9 +232,10 @@ int32_t dtb_device_bytes(dtb_ctx* ctx, int64_t* bytes);
 int32_t dtb_get_stream(dtb_ctx* ctx, void** stream);
 int32_t dtb_sync(dtb_ctx* ctx);
 
-/* Kernel launches issued per step by dtb_run (for launch accounting); the diagnostics
- * reduction adds one launch per sequence of steps (a graph replay, or up to a graph's length
- * of steps run outside one). */
+/* Kernel launches of a step run by itself (for launch accounting); the diagnostics reduction
+ * adds one launch per sequence of steps (a graph replay, or up to a graph's length of steps run
+ * outside one). A run that keeps the gain in shared memory (opts.graph_steps) takes two launches
+ * per sequence in all. */
 int32_t dtb_launches_per_step(dtb_ctx* ctx, int32_t* n);
 /* Kernel launches the context's step functions (dtb_step, dtb_step_io, dtb_run, dtb_solve) have
  * issued so far, kernels replayed in graphs included. No counterpart in the reference. */
