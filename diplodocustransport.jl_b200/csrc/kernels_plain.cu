@@ -237,16 +237,17 @@ int pass_blocks_per_sm(const GainPass& p, int f_smem_len) {
 // take 61 us per step in one pass and 321 us in eight.
 // 16-byte columns per thread: what covers the longest b-row with 256 threads, and with three or more
 // FP64 cells at least two, since every cell costs a broadcast read of f1 per b-row and the columns
-// share it. One FP32 cell takes four where a b-row then still fills a warp: they also share f1's
-// conversion (77 against 85 ms for 64 steps of 2 x 1024 states). On shorter b-rows, and with FP64,
-// more columns cost more in idle threads than they save (40 steps of 2 x 128 FP64 states: 509 us
-// with four, 454 with one; 30 of 140 + 126 FP32 states: 377 with two, 338 with one).
+// share it. One FP32 cell takes four where a b-row then still takes most of a warp (24 threads): they
+// also share f1's conversion (64 steps of 2 x 1024 states: 75 against 83 ms; 19 of 2 x 399: 1.55
+// against 1.68). On shorter b-rows, and with FP64, more columns cost more in idle threads than they
+// save (FP32, 30 steps of 360 + 270 states: 1.39 against 1.40 ms, 40 of 2 x 256: 1.14 against 1.11;
+// FP64, 40 steps of 2 x 128: 0.51 against 0.45).
 GainPass gain_pass(int elem_size, int f_smem_len, int max_n2p, int n_cells) {
     GainPass p;
     const int nvr = max_n2p * elem_size / 16, n = 16 / elem_size;
     p.kv = nvr <= kGainConsumers ? 1 : (nvr <= 2 * kGainConsumers ? 2 : 4);
     if (elem_size == 8 && n_cells > 2) p.kv = std::max(p.kv, 2);
-    if (elem_size == 4 && n_cells == 1 && nvr >= 4 * 32) p.kv = 4;
+    if (elem_size == 4 && n_cells == 1 && nvr >= 96) p.kv = 4;
     int most = std::min(kGainMaxCells, 32 / (p.kv * n));
     if (elem_size == 8 && p.kv == 1) most = std::min(most, 2);
     while (most > 1 && gain_stream_smem_bytes(elem_size, f_smem_len, most) > kGainSmemLimit) --most;
