@@ -106,6 +106,13 @@ struct GainPass {
 };
 constexpr int kGainMaxCells = 8;
 constexpr int kGainSmemLimit = 232448;  // shared memory a CTA may have on sm_100
+// The dynamic shared-memory limit belongs to the kernel instance, which contexts and contractions of
+// different sizes share, and the last value set counts: so it is always set to the most a CTA may
+// have, never to one context's need.
+template <typename Kernel>
+cudaError_t allow_gain_smem(Kernel k) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kGainSmemLimit);
+}
 GainPass gain_pass(int elem_size, int f_smem_len, int max_n2p, int n_cells);
 
 template <typename T>

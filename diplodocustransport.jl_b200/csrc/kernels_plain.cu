@@ -221,7 +221,7 @@ int pass_blocks_per_sm(const GainPass& p, int f_smem_len) {
     int n = 0;
     const int smem = gain_stream_smem_bytes(sizeof(T), f_smem_len, p.cells);
     const auto k = gain_kernel<T>(p);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+    if (smem > kGainSmemLimit || allow_gain_smem(k) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kGainThreads, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -272,7 +272,7 @@ cudaError_t launch_gain_stream(const GainPass& pass, const T* G, const GainUnit*
         so.off[i] = sp_off_host[i];
         so.offp[i] = sp_off_host[n_species + 1 + i];
     }
-    // the dynamic shared-memory limit was raised by gain_stream_blocks_per_sm at commit
+    // the instance's dynamic shared-memory limit was raised by gain_stream_blocks_per_sm
     const int smem = gain_stream_smem_bytes(sizeof(T), f_smem_len, pass.cells);
     const auto k = gain_kernel<T>(pass);
     dim3 grid(grid_x, (n_cells + pass.cells - 1) / pass.cells);

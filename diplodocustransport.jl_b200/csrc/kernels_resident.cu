@@ -434,7 +434,7 @@ int resident_max_states() { return kResStates * kResThreads; }
 template <typename T>
 cudaError_t prepare_resident(const GainPass& p, bool sy, int n_state, int smem, int* blocks_per_sm) {
     const auto k = res_kernel<T>(p, sy, n_state);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_gain_smem(k);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, kResThreads, smem);
 }
