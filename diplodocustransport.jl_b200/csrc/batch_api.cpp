@@ -20,6 +20,7 @@
 
 #include "batch_internal.h"
 #include "ctx.h"
+#include "gemm_plan.h"
 
 namespace dtb {
 
@@ -149,15 +150,6 @@ double ord_dec_host(unsigned long long e) {
 // ---------------------------------------------------------------- gain GEMM plans
 namespace {
 
-// One way to run a group's gain GEMM: the kernel (one SM per tile, or an SM pair sharing a
-// 256 x 256 MMA), the column tile width and the requested number of K splits.
-struct GemmPlan {
-    int pair = 0;
-    int bn = 256;
-    int splits = 1;
-    double us = 0;  // measured time of one GEMM with this plan (0: not measured)
-};
-
 // Plans chosen so far in this process, by shape; a cache file (dtb_set_tune_cache) seeds it and
 // records what the autotuner measures, one line per shape:
 //   sm<SMs>:M<rows>:N1<n1>:n2<n2>:cols<columns>:cells<cells> <pair> <bn> <splits> <us>
@@ -172,68 +164,20 @@ std::string plan_key(const dtb_ctx* c, const MixedGroup& G, int Bcols) {
     return k;
 }
 
-bool plan_valid(const MixedGroup& G, const GemmPlan& p, int max_pairs) {
-    if (p.bn != 64 && p.bn != 128 && p.bn != 256) return false;
-    if (p.splits < 1) return false;
-    if (p.pair && (p.bn != 256 || G.m_tiles % 2 != 0 || max_pairs <= 0)) return false;
-    return true;
+GemmShape gemm_shape(const dtb_ctx* c, const MixedGroup& G, int Bcols, int max_pairs) {
+    return {G.m_tiles, G.n_cb, G.N1, Bcols, c->num_sms, max_pairs};
 }
 
-// Tile counts and K splits of a plan. The splits are aligned to the 64-wide input-2 blocks
-// when that keeps nearly every requested split: a split then never reloads its f2 block in
-// mid-stream.
-void apply_plan(MixedGroup& G, const GemmPlan& p, int Bcols) {
+// Tile counts and K splits of a plan.
+void apply_plan(MixedGroup& G, const GemmShape& g, const GemmPlan& p) {
     G.pair = p.pair != 0;
     G.bn = p.bn;
-    G.n_tiles = (Bcols + p.bn - 1) / p.bn;
+    G.n_tiles = (g.cols + p.bn - 1) / p.bn;
     G.Bpad = G.n_tiles * p.bn;
-    const int T = G.n_cb * G.N1;
-    const int S = std::max(1, std::min(p.splits, T));
-    G.tiles_per_split = (T + S - 1) / S;
-    G.n_splits = (T + G.tiles_per_split - 1) / G.tiles_per_split;
-    const int k_cb = S / G.n_cb;
-    G.splits_per_cb = 0;
-    if (k_cb >= 1 && k_cb <= G.N1 && (double)(k_cb * G.n_cb) >= 0.95 * S) {
-        G.splits_per_cb = k_cb;
-        G.n_splits = k_cb * G.n_cb;
-    }
-}
-
-// Splits that fill the device once: one CTA per SM, or one pair per co-resident cluster.
-// K splits that fill the device once, or a whole number of times (at most kMaxWaves) when one
-// fill would leave a hi*hi accumulator more K tiles than its bound. A GEMM kernel spreads a
-// split's hi*hi products over 512 / bn - 1 tensor-memory accumulators (one on SM pairs). Each is
-// FP32 and its error grows with the number of MMAs it sums (measured: about 2e-5 relative after
-// 3,328 K values in one accumulator; config 3 reached 3e-4 in its state after 5,000 steps with
-// 20,736 K values per accumulator), so the bound keeps the gain term's error at a few 1e-6:
-// 16 K tiles per accumulator on one SM, 32 on SM pairs (where a second fill would double the
-// tensor-bound step's partial traffic).
-constexpr int kMaxTilesPerAccSm = 16;
-constexpr int kMaxTilesPerAccPair = 32;
-constexpr int kMaxWaves = 4;
-constexpr int kShortSplit = 16;  // K tiles: splits this short are also tried longer (tune_group)
-int fill_splits(const dtb_ctx* c, const MixedGroup& G, int pair, int bn, int Bcols, int max_pairs) {
-    const int n_tiles = (Bcols + bn - 1) / bn;
-    const double units = pair ? (double)(G.m_tiles / 2 * n_tiles) : (double)(G.m_tiles * n_tiles);
-    const double cap = pair ? max_pairs : c->num_sms;  // CTAs (pairs) the device runs at once
-    // rounded down: one CTA more than the device holds would run in a second wave on its own
-    const int fill = std::max(1, (int)(cap / units));
-    const int per_split = pair ? kMaxTilesPerAccPair : kMaxTilesPerAccSm * (512 / bn - 1);
-    const int T = G.n_cb * G.N1;
-    const int need = (T + per_split - 1) / per_split;
-    const int waves = std::min(kMaxWaves, std::max(1, (need + fill - 1) / fill));
-    if (waves == 1) return fill;
-    // several waves: as many splits as whole waves hold (the last wave then runs nearly full)
-    return std::max(fill * waves, (int)(waves * cap / units));
-}
-
-// Without timing: the widest tile the columns fill, on SM pairs when the rows pair up.
-GemmPlan heuristic_plan(const dtb_ctx* c, const MixedGroup& G, int Bcols, int max_pairs) {
-    GemmPlan p;
-    p.bn = Bcols >= 192 ? 256 : (Bcols > 64 ? 128 : 64);
-    p.pair = (p.bn == 256 && G.m_tiles % 2 == 0 && max_pairs > 0) ? 1 : 0;
-    p.splits = fill_splits(c, G, p.pair, p.bn, Bcols, max_pairs);
-    return p;
+    const GemmSplits s = gemm_splits(g, p);
+    G.tiles_per_split = s.tiles_per_split;
+    G.n_splits = s.n_splits;
+    G.splits_per_cb = s.per_cb;
 }
 
 }  // namespace
@@ -287,36 +231,17 @@ cudaError_t launch_group_gemm(const dtb_ctx* c, const MixedGroup& G, const float
 // group (every column running, the state at its committed zeros: tensor-core time does not depend
 // on the values; no slot steps, so the epilogue gathers the partials and changes nothing), and
 // returns the fastest. The GEMM alone misleads: more splits mean more partials to gather, and a
-// GEMM that leaves SMs free lets the epilogue's products run beside it. So splits of at most
-// kShortSplit K tiles are also tried half as long again and twice as long. 256 instances on 2 x 128
+// GEMM that leaves SMs free lets the epilogue's products run beside it. 256 instances on 2 x 128
 // states: 17.5 us per step with 128-wide tiles on one SM and 36 splits against 19.6 with the fastest
 // GEMM (SM pairs, 74 splits); 16 instances: 12.5 us with 50 splits against 14.9 with 74.
-int tune_group(dtb_ctx* c, MixedGroup& G, int Bcols, int max_pairs, GemmPlan* best) {
+int tune_group(dtb_ctx* c, MixedGroup& G, const GemmShape& g, GemmPlan* best) {
     MixedState* m = c->mixed;
-    std::vector<GemmPlan> cands;
-    const int T = G.n_cb * G.N1;
-    for (int bn : {64, 128, 256}) {
-        if (bn > 64 && bn / 2 >= Bcols) continue;  // half the tile or more would be padding
-        for (int pair : {0, 1}) {
-            if (pair && (bn != 256 || G.m_tiles % 2 != 0 || max_pairs <= 0)) continue;
-            GemmPlan p;
-            p.bn = bn;
-            p.pair = pair;
-            p.splits = fill_splits(c, G, pair, bn, Bcols, max_pairs);
-            cands.push_back(p);
-            const int fill = p.splits;
-            if (T > kShortSplit * fill) continue;
-            for (int part : {2, 1}) {  // two thirds, half of the splits
-                p.splits = fill * part / (part + 1);
-                if (p.splits >= 1) cands.push_back(p);
-            }
-        }
-    }
-    *best = heuristic_plan(c, G, Bcols, max_pairs);
+    const std::vector<GemmPlan> cands = gemm_plan_candidates(g);
+    *best = gemm_heuristic_plan(g);
     if (cands.size() < 2) return DTB_OK;
     size_t scratch = 0;
     for (const GemmPlan& p : cands) {
-        apply_plan(G, p, Bcols);
+        apply_plan(G, g, p);
         scratch = std::max(scratch, sizeof(float) * (size_t)G.n_splits * G.Bpad * G.M);
     }
     // the timing run's scratch partials and events, released on every way out
@@ -349,12 +274,12 @@ int tune_group(dtb_ctx* c, MixedGroup& G, int Bcols, int max_pairs, GemmPlan* be
             }
         ops.gain_ptr[sp + 1] = e;
     }
-    const int all = Bcols;
+    const int all = g.cols;
     DTB_CUDA(cudaMemcpyAsync(m->active_hi, &all, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     double best_ms = 1e30;
     int rc = DTB_OK;
     for (const GemmPlan& p : cands) {
-        apply_plan(G, p, Bcols);
+        apply_plan(G, g, p);
         G.partial = part;
         set_group_ops(ops, G, gi);
         constexpr int kWarm = 2, kRep = 5;
@@ -402,20 +327,21 @@ int plan_gemms(dtb_ctx* c, int Bcols, int max_pairs) {
     for (auto& G : m->groups) {
         GemmPlan p;
         bool have = false;
+        const GemmShape g = gemm_shape(c, G, Bcols, max_pairs);
         const std::string key = plan_key(c, G, Bcols);
         // held across lookup, tuning and store: concurrent commits of one shape get one plan
         std::unique_lock<std::mutex> lk(g_plan_mu, std::defer_lock);
         if (tune) {
             lk.lock();
             auto it = g_plans.find(key);
-            if (it != g_plans.end() && plan_valid(G, it->second, max_pairs)) {
+            if (it != g_plans.end() && gemm_plan_valid(g, it->second)) {
                 p = it->second;
                 have = true;
             }
         }
         if (!have) {
             if (tune) {
-                DTB_TRY(tune_group(c, G, Bcols, max_pairs, &p));
+                DTB_TRY(tune_group(c, G, g, &p));
                 g_plans[key] = p;
                 if (!g_plan_file.empty()) {
                     if (FILE* f = std::fopen(g_plan_file.c_str(), "a")) {
@@ -424,10 +350,10 @@ int plan_gemms(dtb_ctx* c, int Bcols, int max_pairs) {
                     }
                 }
             } else {
-                p = heuristic_plan(c, G, Bcols, max_pairs);
+                p = gemm_heuristic_plan(g);
             }
         }
-        apply_plan(G, p, Bcols);
+        apply_plan(G, g, p);
         G.tuned_us = p.us;
         DTB_TRY(c->alloc(&G.partial, sizeof(float) * (size_t)G.n_splits * G.Bpad * G.M));
     }
