@@ -26,14 +26,25 @@
 namespace dtb {
 
 // ------------------------------------------------------------------ gain_stream
-// Reduction ring: a consumer warp can run at most kGainStages tiles (hence units) ahead of
-// warp 0, so kGainStages + 2 slots never alias a slot warp 0 is still reading.
-constexpr int kRedRing = kGainStages + 2;
+// Ring of the units in flight in a block (records and warp sums). A tile is copied once every
+// consumer warp has released the tile kGainStages before it, and a unit has at least one tile: when
+// a unit's record is written, or its warp sums are, every warp is past the unit kGainStages + 1
+// before it, so that many slots never alias one still read.
+constexpr int kRedRing = kGainStages + 1;
+
+// What the consumers need of a work unit: 16 bytes, so that the ring takes no more shared memory
+// than it leaves to the longest state vectors (20,800 FP64 states). The loop bounds stay 32 bits
+// wide: with 16-bit ones the compiler unrolls the b-rows further, at 3 to 10 % of a step.
+struct GainRec {
+    unsigned short b_off, c_off;
+    int nb, n2p, tile_b;
+};
+static_assert(sizeof(GainRec) == 16, "GainRec layout");
 
 int gain_stream_smem_bytes(int elem_size, int f_smem_len, int cells) {
     return kGainStages * kGainTileBytes + round_up_int(f_smem_len * cells * (cells == 1 ? elem_size : 8), 16) +
-           2 * kGainStages * 8 + kRedRing * 8 + kRedRing * (int)sizeof(GainUnit) +
-           kRedRing * kGainConsumerWarps * cells * 8 + 16;
+           2 * kGainStages * 8 + kRedRing * 8 + kRedRing * (int)sizeof(GainRec) +
+           kRedRing * kGainConsumerWarps * cells * 8 + 8;
 }
 
 // One block streams work units through a ring of 16 KB tiles for up to C space cells at once
@@ -58,7 +69,7 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
                                                  round_up_int(f_len * C * (int)sizeof(S), 16));
     uint64_t* empty = full + kGainStages;
     uint64_t* unit_bar = empty + kGainStages;
-    GainUnit* unit_s = reinterpret_cast<GainUnit*>(unit_bar + kRedRing);  // the work records, by unit slot
+    GainRec* unit_s = reinterpret_cast<GainRec*>(unit_bar + kRedRing);  // by unit slot
     double* red = reinterpret_cast<double*>(unit_s + kRedRing);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(red + kRedRing * kGainConsumerWarps * C);
 
@@ -77,7 +88,8 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
     }
     __syncthreads();  // barriers initialised; the producer may stream G before f is ready
     const auto bad = [](const GainUnit& U) {
-        return U.nb <= 0 || U.tile_b <= 0 || U.n2p <= 0 || U.tile_b * U.n2p > kTileElems || U.n2p / Vec<T>::n > kMaxVec;
+        return U.nb <= 0 || U.tile_b <= 0 || U.n2p <= 0 || U.tile_b * U.n2p > kTileElems ||
+               U.n2p / Vec<T>::n > kMaxVec || (unsigned)U.b_off > 65535u || (unsigned)U.c_off > 65535u;
     };
 
     if (warp == kGainConsumerWarps) {
@@ -106,9 +118,9 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
                         ok = false;
                         break;
                     }
-                    // the record reaches the consumers with the unit's first tile; its slot is free:
-                    // a unit kRedRing back was reduced before this stage was released
-                    if (t == 0) unit_s[lk % kRedRing] = U;
+                    // the record reaches the consumers with the unit's first tile
+                    if (t == 0)
+                        unit_s[lk % kRedRing] = {(unsigned short)U.b_off, (unsigned short)U.c_off, U.nb, U.n2p, U.tile_b};
                     const int rows = min(U.tile_b, U.nb - t * U.tile_b);
                     const uint32_t bytes = (uint32_t)rows * (uint32_t)U.n2p * (uint32_t)sizeof(T);
                     mbar_arrive_expect_tx(smem_u32(&full[st]), bytes);
@@ -140,7 +152,7 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
     int c_off = -1, n2p = 0;  // the columns in sum's x
     for (int u = blockIdx.x; u < n_units; u += gridDim.x, ++lk) {
         const int slot = lk % kRedRing;
-        const GainUnit* U = &unit_s[slot];  // valid from the unit's first tile on
+        const GainRec* U = &unit_s[slot];  // valid from the unit's first tile on
         UnitMap m{};
         const S* f1 = f_s;
         sum.begin();
