@@ -1827,7 +1827,9 @@ int32_t dtb_selftest_bounded_wait(dtb_ctx* c, double limit_s) {
 int32_t dtb_gain_kernel_stats(dtb_ctx* c, double* avg_ms, double* bytes_per_launch) {
     DTB_CHECK(c, DTB_EINVAL, "dtb_gain_kernel_stats: null context");
     DTB_TRY(dtb_commit(c));
-    if (bytes_per_launch) *bytes_per_launch = c->gain_bytes * c->n_bin_cells;
+    // a launch reads G once per pass over its cells (grid y of gain_stream)
+    const int per = std::max(1, c->gain_pass.cells);
+    if (bytes_per_launch) *bytes_per_launch = c->gain_bytes * ((c->n_bin_cells + per - 1) / per);
     if (avg_ms) *avg_ms = c->prof_n ? c->prof_ms / (double)c->prof_n : 0.0;
     return DTB_OK;
 }

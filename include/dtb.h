@@ -247,7 +247,8 @@ int32_t dtb_launch_count(dtb_ctx* ctx, int64_t* n);
 int32_t dtb_selftest_bounded_wait(dtb_ctx* ctx, double limit_s);
 
 /* Dominant-kernel timing over the last dtb_run: average gain-kernel duration in ms measured
- * with CUDA events on the context stream, and its algorithmic bytes per launch. */
+ * with CUDA events on the context stream, and its algorithmic bytes per launch (one read of the gain
+ * blocks for every eight space cells or fewer that share it). */
 int32_t dtb_gain_kernel_stats(dtb_ctx* ctx, double* avg_ms, double* bytes_per_launch);
 int32_t dtb_set_profiling(dtb_ctx* ctx, int32_t on);
 
