@@ -550,28 +550,19 @@ static void sparse_runs(const SparseGain& g, int64_t n2p, int64_t max_elems, std
 }
 
 // Whether runs may use the kernel that keeps the gain units in shared memory: the library's choice
-// of how to run steps (opts.graph_steps 0), every cell in the binary domain, and a state that one
-// block can update.
-static bool resident_eligible(const dtb_ctx* c) {
+// of how to run steps (opts.graph_steps 0), every cell in the binary domain, a state that one block
+// can update, and an X flux (space pass of the symplectic method) of few slots.
+static bool resident_eligible(const dtb_ctx* c, int x_ell_w) {
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
     return coop && c->opts.graph_steps == 0 && c->n_bin_cells == c->n_space && !c->has_bin_domain &&
-           c->n_state <= resident_max_states();
+           c->n_state <= resident_max_states() && (!c->symplectic || x_ell_w <= kResMaxX);
 }
 
-// Device arrays of that kernel, once the flux is known.
-template <typename T>
-static int commit_resident(dtb_ctx* c, const RowOps<T>& ops, const std::vector<int>& first,
-                           const std::vector<int>& own, const std::vector<int>& slot) {
+// Device arrays of that kernel.
+static int commit_resident(dtb_ctx* c, const std::vector<int>& first, const std::vector<int>& own,
+                           const std::vector<int>& slot) {
     if (!c->res_on) return DTB_OK;
-    int bps = 0;
-    const bool fits = (!c->symplectic || ops.x_ell_w <= kResMaxX) &&
-                      prepare_resident<T>(c->res_pass, c->symplectic, (int)c->n_state, c->res_smem, &bps) == cudaSuccess && bps >= 1;
-    if (!fits) {
-        cudaGetLastError();
-        c->res_on = false;
-        return DTB_OK;
-    }
     ResidentArgs& r = c->res;
     int *d_first, *d_own, *d_slot;
     DTB_TRY(copy_host_ints(c, &d_first, first));
@@ -711,6 +702,18 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
             g.host.shrink_to_fit();
         }
     }
+    // ---------------- flux: CSR with duplicates summed, then banded ELL (X + P, or P and X
+    // separately for the symplectic method)
+    DTB_TRY(build_ell<T>(c, c->flux_r, c->flux_c, c->flux_v, ops.ell_w, ops.ell_val, ops.ell_col));
+    if (c->symplectic) {
+        DTB_TRY(build_ell<T>(c, c->xflux_r, c->xflux_c, c->xflux_v, ops.x_ell_w, ops.x_ell_val, ops.x_ell_col));
+        T *fm, *dfm;
+        DTB_TRY(c->alloc(&fm, sizeof(T) * (size_t)c->n_state));
+        DTB_TRY(c->alloc(&dfm, sizeof(T) * (size_t)c->n_state));
+        c->fm_buf = fm;
+        c->dfm_buf = dfm;
+        ops.dfm_out = dfm;
+    }
     // binary domain: `in(off_space, Domain)` per cell (entries outside 0..n_space-1 match no cell)
     ops.bin_on = nullptr;
     c->n_bin_cells = c->n_space;
@@ -796,8 +799,13 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
         // plus, per unit, about what a unit's reduction costs in streaming time. At most about 32
         // units per CTA are looked at. (Against eight units per CTA whatever the remainder: 44.3
         // against 46.4 us per step on one cell of 2 x 256 FP64 states, 61 against 71 on eight.)
+        // A G that L2 holds streams at about 160 KB per us and CTA, and a unit's round trip of
+        // about 0.9 us is hardly hidden: whole rows where there are enough of them. Per step, units
+        // of 16 KB, 64 KB and whole rows: 2 x 128 FP64 states 10.0, 8.4 and 7.4 us, 24 + 384 FP64
+        // 10.3, 9.7 and 8.1, 2 x 128 FP32 8.4, 7.5 and 7.4.
         const size_t ctas = (size_t)c->num_sms * bps;
-        const double unit_cost = 4096.0 + 1024.0 * c->gain_pass.cells;
+        const bool in_l2 = tot_bytes <= 64.0 * 1024 * 1024;
+        const double unit_cost = in_l2 ? 128.0 * 1024 : 4096.0 + 1024.0 * c->gain_pass.cells;
         double target = kGainTileBytes, best = 0;
         std::vector<double> load(ctas);
         for (double t = 256.0 * 1024; t >= kGainTileBytes; t -= t > 128.0 * 1024 ? 32768 : 16384) {
@@ -816,8 +824,12 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
         }
         // A grid whose units fit the SMs' shared memory is planned for the kernel that keeps them
         // there: the units in order, cut into one run of nearly equal bytes per SM, judged by the
-        // fullest group of threads of a block.
-        if (resident_eligible(c)) {
+        // fullest group of threads of a block. In that a unit counts as much as 24 KB beside its
+        // bytes, and so does a row cut between blocks, whose segments wait for one another in every
+        // step (2 x 112 FP64 states: 4.1 us per step with whole rows, 4.9 with two units per row, 6.4
+        // with seven; 24 + 384 FP64: 4.9 with whole rows, 6.8 with five units per row).
+        const double stream_target = target;
+        if (resident_eligible(c, ops.x_ell_w)) {
             c->res_pass = resident_pass((int)esz, c->gain_pass, c->n_space);
             const bool pad = c->offp[c->ns] != c->n_mom;
             double res_best = 0;
@@ -826,7 +838,7 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
                 each_unit(t, [&](const GainUnit& w) { list.push_back({w.row, (int64_t)w.nb * w.n2p * (int64_t)esz}); });
                 const size_t n = list.size(), grid = std::min<size_t>(n, (size_t)c->num_sms);
                 if (n == 0 || n > grid * 256) break;
-                const double cost = 4096;  // what a unit costs beside its bytes
+                const double cost = 4096, price = 24.0 * 1024;
                 double total = 0, cum = 0;
                 for (auto& w : list) total += (double)w.second + cost;
                 std::vector<int> first(grid + 1, (int)n), own(grid + 1, (int)c->n_mom), slot(n, 0);
@@ -844,7 +856,7 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
                             blk + 1 == grid)) {
                         cum += (double)list[u].second + cost;
                         bytes[blk] += list[u].second;
-                        part[(u - (size_t)first[blk]) % kResGroups] += (double)list[u].second + cost;
+                        part[(u - (size_t)first[blk]) % kResGroups] += (double)list[u].second + price;
                         if (u > 0 && list[u].first == list[u - 1].first)
                             slot[u] = slot[u - 1] + (u == (size_t)first[blk] ? 1 : 0);
                         segs = std::max(segs, slot[u] + 1);
@@ -864,6 +876,7 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
                 const int smem = resident_smem_bytes(c->res_pass, (int)esz, (int)g, (int)c->offp[c->ns], c->n_space,
                                                      (int)c->n_state, pad, max_local, max_own);
                 if (smem > kGainSmemLimit) continue;
+                if (segs > 1) group += price;
                 if (!c->res_on || group < res_best) {
                     res_best = group;
                     target = t;
@@ -879,6 +892,14 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
                     res_slot.swap(slot);
                 }
             }
+        }
+        int res_bps = 0;
+        if (c->res_on && (prepare_resident<T>(c->res_pass, c->symplectic, (int)c->n_state, c->res_smem, &res_bps) !=
+                              cudaSuccess ||
+                          res_bps < 1)) {
+            cudaGetLastError();
+            c->res_on = false;
+            target = stream_target;
         }
         each_unit(target, [&](const GainUnit& u) {
             while (unit_row < u.row) unit_ptr[(size_t)++unit_row] = (int)units.size();
@@ -992,18 +1013,6 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
         ops.emi_ncols = d_nc;
         ops.emi_data = d_data;
     }
-    // ---------------- flux: CSR with duplicates summed, then banded ELL (X + P, or P and X
-    // separately for the symplectic method)
-    DTB_TRY(build_ell<T>(c, c->flux_r, c->flux_c, c->flux_v, ops.ell_w, ops.ell_val, ops.ell_col));
-    if (c->symplectic) {
-        DTB_TRY(build_ell<T>(c, c->xflux_r, c->xflux_c, c->xflux_v, ops.x_ell_w, ops.x_ell_val, ops.x_ell_col));
-        T *fm, *dfm;
-        DTB_TRY(c->alloc(&fm, sizeof(T) * (size_t)c->n_state));
-        DTB_TRY(c->alloc(&dfm, sizeof(T) * (size_t)c->n_state));
-        c->fm_buf = fm;
-        c->dfm_buf = dfm;
-        ops.dfm_out = dfm;
-    }
     ops.mode = 0;
     ops.thr_mom = c->prec == DTB_F64 ? (double)1e-10f : (double)(T)1e-10f;
     ops.thr_space = c->prec == DTB_F64 ? (double)1e-20f : (double)(T)1e-20f;
@@ -1043,7 +1052,7 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
     ops.thr = c->prec == DTB_F64 ? (double)1e-10f : (double)(T)1e-10f;
     ops.has_bin = c->has_bin;
     ops.has_emi = c->has_emi;
-    return commit_resident<T>(c, ops, res_first, res_own, res_slot);
+    return commit_resident(c, res_first, res_own, res_slot);
 }
 
 extern "C" int32_t dtb_commit(dtb_ctx* c) {
@@ -1194,6 +1203,15 @@ static int run_loose(dtb_ctx* c, int64_t n, int verbose, bool profile) {
     return DTB_OK;
 }
 
+// Steps that pay for loading the units into shared memory. A Solve's save interval does from about
+// four on (five symplectic FP32 cells 93 against 95 us with the host's part, 2 x 128 FP64 72 against
+// 73) and is clearly faster at eight (143 against 160, 87 against 110). dtb_run keeps to the length
+// of a graph, two kernels a step below it: what dtb_launch_count reports for such runs is fixed.
+constexpr int64_t kResMinSteps = 8;
+static bool use_resident(const dtb_ctx* c, int64_t n, int64_t least) {
+    return c->res_on && !c->profiling && n >= least;
+}
+
 // n steps of the resident kernel, a launch per sequence of at most graph_steps (the record slots).
 template <typename T>
 static int run_resident_typed(dtb_ctx* c, const RowOps<T>& ops, int64_t n, int verbose) {
@@ -1269,8 +1287,8 @@ static int run_chunk(dtb_ctx* c, int64_t n, int verbose, bool use_graph) {
     DTB_CUDA(cudaMemsetAsync(c->ctr, 0, sizeof(unsigned long long), c->stream));
     c->host_ctr = 0;
     int64_t done = 0;
-    if (use_graph && c->res_on && !c->profiling && n >= c->graph_steps) return run_resident(c, n, verbose);
-    if (use_graph && !c->profiling && n >= c->graph_steps) {
+    if (use_graph && use_resident(c, n, c->graph_steps)) return run_resident(c, n, verbose);
+    if (use_graph && !c->res_on && !c->profiling && n >= c->graph_steps) {
         if (c->cur != 0) {
             DTB_TRY(run_loose(c, 1, verbose, false));
             done++;
@@ -1527,14 +1545,11 @@ static int ensure_pipe(dtb_ctx* c) {
     return DTB_OK;
 }
 
-// Save intervals of this many steps and more pay for loading the units into shared memory.
-constexpr int64_t kResMinSteps = 8;
-
 // n steps through the device counter from its current value (the resident kernel or graph replays
 // where they fit).
 static int run_steps(dtb_ctx* c, int64_t n, int verbose) {
     int64_t done = 0;
-    if (c->res_on && !c->profiling && n >= kResMinSteps) return run_resident(c, n, verbose);
+    if (use_resident(c, n, kResMinSteps)) return run_resident(c, n, verbose);
     if (!c->res_on && !c->profiling && n >= c->graph_steps) {
         if (c->cur != 0) {
             DTB_TRY(run_loose(c, 1, verbose, false));

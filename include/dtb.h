@@ -72,10 +72,12 @@ typedef struct dtb_opts {
     int32_t graph_steps;   /* steps per captured CUDA graph (at most 1024). 0: the default, for
                               plain contexts 64 when the step records of 64 steps fit in 8 MB
                               (grids up to about 175,000 states) and 16 above; 16 for batched
-                              ones. 0 also lets longer runs of a plain context on a small grid
-                              (gain blocks up to about 33 MB) keep the gain in shared memory, one
-                              launch for 64 steps, with the same results bit for bit; any other
-                              value keeps two launches per step */
+                              ones. 0 also lets a plain context on a small grid (gain blocks up to
+                              about 33 MB) keep the gain in shared memory, one launch for 64 steps,
+                              in runs of 64 steps and more and in a Solve's save intervals of eight
+                              and more, with the bits of the same context's steps run one by one.
+                              Any other value keeps two launches per step, and may sum the gain in
+                              other units, so that the last bits differ from those under 0 */
     double dt0;            /* TimeStruct.dt0 (StructsAndDictionaries.jl:55) */
     int32_t batch;         /* instances per context; 1 for the plain method */
     int32_t flags;         /* reserved, 0 */
