@@ -739,7 +739,9 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
     for (auto& b : blks) max_n2p = std::max(max_n2p, (int)b.n2p);
     for (auto& sb : sblks)
         for (auto& R : sb.runs) max_n2p = std::max(max_n2p, R.w);
-    c->gain_pass = gain_pass((int)esz, c->f_smem_len, max_n2p, std::max(1, c->n_bin_cells));
+    double tot_bytes = sparse_bytes;
+    for (auto& b : blks) tot_bytes += (double)b.no * b.n1 * b.n2 * esz;
+    c->gain_pass = gain_pass((int)esz, c->f_smem_len, max_n2p, std::max(1, c->n_bin_cells), tot_bytes, kFourColsStep);
     int bps = gain_stream_blocks_per_sm((int)esz, c->gain_pass, c->f_smem_len);
     DTB_CHECK(bps >= 1 || (blks.empty() && sblks.empty()), DTB_EINVAL,
               "gain kernel does not fit on an SM (state vector too long)");
@@ -749,8 +751,6 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
     int unit_row = 0;
     std::vector<int> res_first, res_own, res_slot;
     {
-        double tot_bytes = sparse_bytes;
-        for (auto& b : blks) tot_bytes += (double)b.no * b.n1 * b.n2 * esz;
         c->gain_bytes = tot_bytes;
         // sparse runs per output row (global momentum index)
         std::vector<std::vector<std::pair<const SpBlk*, const SparseRun*>>> srow((size_t)c->n_mom);

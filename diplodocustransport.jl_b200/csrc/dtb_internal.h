@@ -113,7 +113,10 @@ template <typename Kernel>
 cudaError_t allow_gain_smem(Kernel k) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kGainSmemLimit);
 }
-GainPass gain_pass(int elem_size, int f_smem_len, int max_n2p, int n_cells);
+// Bytes of G above which one FP32 cell takes four columns per thread: in a step, whose other kernels
+// leave L2 to G, in a single contraction, and on wide b-rows.
+constexpr double kFourColsStep = 150e6, kFourColsOp = 80e6, kFourColsWide = 48e6;
+GainPass gain_pass(int elem_size, int f_smem_len, int max_n2p, int n_cells, double g_bytes, double four_from);
 
 template <typename T>
 cudaError_t launch_gain_stream(const GainPass& pass, const T* G, const GainUnit* units, int n_units, const T* f,
@@ -217,6 +220,8 @@ struct GainOpPlan {
     int64_t nb;
     int tile_b;
 };
+// CTAs per SM of the pass a contraction takes (0: its vectors are too long)
+int gain_op_blocks_per_sm(int64_t n_out, int64_t n1, int64_t n2, int esz);
 int gain_op_plan(int64_t n_out, int64_t n1, int64_t n2, int esz, int num_sms, int bps, GainOpPlan& plan);
 int gain_op_run(int32_t dtype, const void* G, int64_t n_out, int64_t n1, int64_t n2, const void* f1, const void* f2,
                 double* out, const GainOpPlan& plan, unsigned char* scratch, int* err, cudaStream_t s);

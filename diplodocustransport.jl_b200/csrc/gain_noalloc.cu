@@ -67,9 +67,7 @@ extern "C" int32_t dtb_gain_contract_noalloc(int32_t dtype, const void* G, int64
     }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     GainOpPlan plan;
-    const int f_len = (int)((n1 + 7) / 8 * 8 + n2);
-    rc = gain_op_plan(n_out, n1, n2, esz, sms, gain_stream_blocks_per_sm(esz, gain_pass(esz, f_len, (int)n2, 1), f_len),
-                      plan);
+    rc = gain_op_plan(n_out, n1, n2, esz, sms, gain_op_blocks_per_sm(n_out, n1, n2, esz), plan);
     if (rc != DTB_OK) return rc;
     if (plan.n_units > kNoallocMaxUnits) {
         set_error("dtb_gain_contract_noalloc: the block needs " + std::to_string(plan.n_units) +

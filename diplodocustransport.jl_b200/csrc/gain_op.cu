@@ -48,6 +48,13 @@ __global__ void gain_op_units_kernel(GainUnit* __restrict__ units, long long n_u
     units[u] = g;
 }
 
+static GainPass gain_op_pass(int64_t n_out, int64_t n1, int64_t n2, int esz) {
+    return gain_pass(esz, (int)((n1 + 7) / 8 * 8 + n2), (int)n2, 1, (double)n_out * n1 * n2 * esz, kFourColsOp);
+}
+int gain_op_blocks_per_sm(int64_t n_out, int64_t n1, int64_t n2, int esz) {
+    return gain_stream_blocks_per_sm(esz, gain_op_pass(n_out, n1, n2, esz), (int)((n1 + 7) / 8 * 8 + n2));
+}
+
 int gain_op_plan(int64_t n_out, int64_t n1, int64_t n2, int esz, int num_sms, int bps, GainOpPlan& plan) {
     const int64_t row_b = n2 * esz;
     if (n2 <= 0 || n2 % 8 != 0 || row_b > kGainTileBytes) {
@@ -145,7 +152,7 @@ int gain_op_run(int32_t dtype, const void* G, int64_t n_out, int64_t n1, int64_t
     int sp[6] = {0, (int)n1, (int)(n1 + n2), 0, (int)offp1, (int)(offp1 + n2)};
     const int f_len = (int)(offp1 + n2);
     const int n_state = (int)(n1 + n2);
-    const GainPass pass = gain_pass(esz, f_len, (int)n2, 1);
+    const GainPass pass = gain_op_pass(n_out, n1, n2, esz);
     const int bps = gain_stream_blocks_per_sm(esz, pass, f_len);
     if (bps < 1) {
         set_error("gain op: vectors too long for the shared-memory stage");
@@ -210,9 +217,7 @@ extern "C" int32_t dtb_gain_contract(int32_t dtype, const void* G, int64_t n_out
     }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     GainOpPlan plan;
-    const int f_len = (int)((n1 + 7) / 8 * 8 + n2);
-    rc = gain_op_plan(n_out, n1, n2, esz, sms, gain_stream_blocks_per_sm(esz, gain_pass(esz, f_len, (int)n2, 1), f_len),
-                      plan);
+    rc = gain_op_plan(n_out, n1, n2, esz, sms, gain_op_blocks_per_sm(n_out, n1, n2, esz), plan);
     if (rc != DTB_OK) return rc;
     const size_t need = gain_op_scratch_bytes(plan.n_units, n1, n2, esz);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);

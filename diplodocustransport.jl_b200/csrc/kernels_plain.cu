@@ -225,7 +225,8 @@ GainKernel<T> gain_kernel(const GainPass& p) {
     constexpr int n = Vec<T>::n;
     if (p.kv == 1) return gain_kernel_upto<T, 1, sizeof(T) == 8 ? 2 : 8>(p.cells);
     if (p.kv == 2) return gain_kernel_upto<T, 2, 32 / (2 * n)>(p.cells);
-    return gain_kernel_upto<T, 4, 32 / (4 * n)>(p.cells);
+    if constexpr (sizeof(T) == 8) return gain_kernel_upto<T, 4, 4>(p.cells);
+    return p.kv == 3 ? gain_stream_kernel<T, 1, 3> : gain_stream_kernel<T, 1, 4>;
 }
 
 template <typename T>
@@ -246,22 +247,34 @@ int pass_blocks_per_sm(const GainPass& p, int f_smem_len) {
 // Cells that share one read of G: as many as fit a thread's accumulators (32 FP64 values, 8 cells
 // at most) and the staged states a CTA's shared memory, split evenly over the passes they take
 // (the least padding). G is the traffic: eight cells of a 2 x 256-state FP64 grid (268 MB of G)
-// take 61 us per step in one pass and 321 us in eight.
+// take 61 us per step in one pass and 321 us in eight. Four columns per thread spill at the most
+// cells: with FP32 a pass takes one cell then (b-rows of 2,056 states, two cells: 86 us per step in
+// two passes, 144 in one), with FP64 three, or just four where the threads' last column is nearly
+// full (b-rows of 1,032 / 1,600 / 2,000 states: four cells in two passes 41 / 85 / 122 us, in one
+// 75 / 87 / 110; eight in three passes 76 / 138 / 194, in two 127 / 167 / 212).
 // 16-byte columns per thread: what covers the longest b-row with 256 threads, and with three or more
 // FP64 cells at least two, since every cell costs a broadcast read of f1 per b-row and the columns
-// share it. One FP32 cell takes four where a b-row then still takes most of a warp (24 threads): they
-// also share f1's conversion (64 steps of 2 x 1024 states: 75 against 83 ms; 19 of 2 x 399: 1.55
-// against 1.68). On shorter b-rows, and with FP64, more columns cost more in idle threads than they
-// save (FP32, 30 steps of 360 + 270 states: 1.39 against 1.40 ms, 40 of 2 x 256: 1.14 against 1.11;
-// FP64, 40 steps of 2 x 128: 0.51 against 0.45).
-GainPass gain_pass(int elem_size, int f_smem_len, int max_n2p, int n_cells) {
+// share it. One FP32 cell takes four: they also share f1's conversion to FP64, and a tile is one
+// round of the block. That pays where G comes from HBM (kFourColsStep, kFourColsOp: 30 steps of
+// 2 x 328 and 2 x 352 states 1.48 and 1.73 against 1.52 and 1.83 ms, 8 of 2 x 1024 9.5 against 10.5;
+// contractions of 268 to 540 MB 4 to 8 % faster), or on b-rows of 96 columns and more from a G of some size (30 steps of
+// 128 + 384 states, 101 MB: 0.60 against 0.67 ms); not from a G that L2 serves (2 x 232 states,
+// 100 MB: 0.79 against 0.68 ms; 32 + 480, 31 MB: 0.40 against 0.36), nor on rows of a few columns
+// (2048 x 2048 x 16: 83 against 66 us). Rows of 513 to 768 columns take three: 5 % faster than four.
+// With FP64 more columns cost more in idle threads than they save (40 steps of 2 x 128: 0.51
+// against 0.45 ms).
+GainPass gain_pass(int elem_size, int f_smem_len, int max_n2p, int n_cells, double g_bytes, double four_from) {
     GainPass p;
     const int nvr = max_n2p * elem_size / 16, n = 16 / elem_size;
     p.kv = nvr <= kGainConsumers ? 1 : (nvr <= 2 * kGainConsumers ? 2 : 4);
     if (elem_size == 8 && n_cells > 2) p.kv = std::max(p.kv, 2);
-    if (elem_size == 4 && n_cells == 1 && nvr >= 96) p.kv = 4;
+    if (elem_size == 4 && n_cells == 1) {
+        if ((nvr >= 10 && g_bytes > four_from) || (nvr >= 96 && g_bytes > kFourColsWide)) p.kv = 4;
+        if (nvr > 2 * kGainConsumers && nvr <= 3 * kGainConsumers) p.kv = 3;
+    }
     int most = std::min(kGainMaxCells, 32 / (p.kv * n));
     if (elem_size == 8 && p.kv == 1) most = std::min(most, 2);
+    if (p.kv == 4) most = elem_size == 4 ? 1 : (n_cells == 4 && nvr >= 864 ? 4 : 3);
     while (most > 1 && gain_stream_smem_bytes(elem_size, f_smem_len, most) > kGainSmemLimit) --most;
     const int passes = (n_cells + most - 1) / most;
     p.cells = passes > 0 ? (n_cells + passes - 1) / passes : 1;

@@ -168,14 +168,14 @@ __device__ __forceinline__ UnitMap unit_map(int n2p, int tid) {
 }
 
 // A thread's contraction of a work unit, FP64 throughout (the unit is read once for all C cells).
-// With four columns per thread (few cells) the thread keeps its columns' f2 in x and forms
+// With three or four columns per thread (few cells) the thread keeps its columns' f2 in x and forms
 //   acc += f1[b] (g . x) per b-row,
 // so a unit costs no f2 reads of its own while the next one has the same columns; with fewer
 // columns (many cells) it accumulates y += f1[b] g per column and dots with f2 once per unit, which
 // holds one value per column and cell instead of one plus one per cell.
 template <typename T, int C, int KV>
 struct UnitSum {
-    static constexpr bool kDotRows = KV == 4;
+    static constexpr bool kDotRows = KV >= 3;
     using V = Vec<T>;
     using S = typename StagedT<T, C>::type;
     using vec_t = typename V::type;
@@ -230,7 +230,7 @@ struct UnitSum {
             for (int c = 0; c < C; ++c) {
                 const double x1 = (double)f1[c * f_len + r];
                 if constexpr (kDotRows) {
-                    double d[2] = {0.0, 0.0};  // two chains: columns 0, 1 and 2, 3
+                    double d[2] = {0.0, 0.0};  // two chains: columns 0, 1 and the others
 #pragma unroll
                     for (int k = 0; k < KV; ++k)
 #pragma unroll
