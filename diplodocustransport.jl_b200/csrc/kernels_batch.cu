@@ -808,6 +808,7 @@ constexpr int kOP = kCK + 8;      // BF16 row pitch of a staged operand chunk (2
 constexpr int kRowStages = 3;     // cp.async ring depth
 constexpr int kEllFast = 8;       // ELL widths up to this take the hoisted-load flux path
 constexpr int kGatherVec = 18;    // 16-byte split partials in flight per thread in the gain gather
+constexpr int kGatherRow = 8;    // the same where a thread's four rows need a load each
 
 // A tile of RT rows x IT instances on NW warps.
 template <int RT, int IT, int NW>
@@ -1138,14 +1139,24 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) mixed_rows_kernel(MixedRowOp
                         }
                     }
                 }
-            } else if (okv) {
+            } else if (okv) {  // rows that start elsewhere: 4-byte loads, kGatherRow splits of them in flight
                 const int nr = min(4, Mg - (row0 + 4 * rg));
-                for (int c = sp_lo; c < sp_hi; ++c) {
-                    const float* p = pp + (size_t)c * st;
-                    acc.x += p[0];
-                    if (nr > 1) acc.y += p[1];
-                    if (nr > 2) acc.z += p[2];
-                    if (nr > 3) acc.w += p[3];
+                for (int c0 = sp_lo; c0 < sp_hi; c0 += kGatherRow) {
+                    float v[kGatherRow][4];
+#pragma unroll
+                    for (int k = 0; k < kGatherRow; ++k)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            v[k][j] = c0 + k < sp_hi && j < nr ? pp[(size_t)(c0 + k) * st + j] : 0.f;
+#pragma unroll
+                    for (int k = 0; k < kGatherRow; ++k) {
+                        if (c0 + k < sp_hi) {
+                            acc.x += v[k][0];
+                            acc.y += v[k][1];
+                            acc.z += v[k][2];
+                            acc.w += v[k][3];
+                        }
+                    }
                 }
             }
             s_part[h][4 * rg][il] = acc.x;
