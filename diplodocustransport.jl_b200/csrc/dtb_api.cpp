@@ -829,8 +829,8 @@ static int commit_typed(dtb_ctx* c, RowOps<T>& ops) {
         // step (2 x 112 FP64 states: 4.1 us per step with whole rows, 4.9 with two units per row, 6.4
         // with seven; 24 + 384 FP64: 4.9 with whole rows, 6.8 with five units per row).
         const double stream_target = target;
-        if (resident_eligible(c, ops.x_ell_w)) {
-            c->res_pass = resident_pass((int)esz, c->gain_pass, c->n_space);
+        c->res_pass = resident_pass((int)esz, c->gain_pass, c->n_space);
+        if (c->res_pass.cells > 0 && resident_eligible(c, ops.x_ell_w)) {
             const bool pad = c->offp[c->ns] != c->n_mom;
             double res_best = 0;
             for (double t = 256.0 * 1024; t >= kGainTileBytes; t -= t > 128.0 * 1024 ? 32768 : 16384) {

@@ -392,21 +392,32 @@ using ResKernel = void (*)(RowOps<T>, ResidentArgs, SpOff, const T*, T*, const d
 // At most kResAcc accumulators per thread (96 registers).
 constexpr int kResAcc = 24;
 
+// The instances that a state of at most resident_max_states() can ask for. Rows of more than 512
+// FP64 or 1,024 FP32 states leave room for one cell (two with 513 to 960 FP64 states), and a state
+// with them is longer than 640, except one cell's of 513 to 632 FP64 states.
 template <typename T, int KV, int C>
 ResKernel<T> res_kernel_upto(int cells, bool sy, bool one) {
     if constexpr (C > 1) {
         if (cells < C) return res_kernel_upto<T, KV, C - 1>(cells, sy, one);
     }
-    return sy ? (one ? resident_kernel<T, C, KV, true, 1> : resident_kernel<T, C, KV, true, kResStates>)
-              : (one ? resident_kernel<T, C, KV, false, 1> : resident_kernel<T, C, KV, false, kResStates>);
+    if constexpr (KV == 1 || (KV == 2 && sizeof(T) == 8 && C != 2)) {
+        if (one) return sy ? resident_kernel<T, C, KV, true, 1> : resident_kernel<T, C, KV, false, 1>;
+    }
+    return sy ? resident_kernel<T, C, KV, true, kResStates> : resident_kernel<T, C, KV, false, kResStates>;
 }
 template <typename T>
 ResKernel<T> res_kernel(const GainPass& p, bool sy, int n_state) {
     constexpr int n = Vec<T>::n;
     const bool one = n_state <= kResThreads;
-    if (p.kv == 1) return res_kernel_upto<T, 1, sizeof(T) == 8 ? 2 : kResAcc / n>(p.cells, sy, one);
-    return p.kv == 2 ? res_kernel_upto<T, 2, kResAcc / (2 * n)>(p.cells, sy, one)
-                     : res_kernel_upto<T, 4, kResAcc / (4 * n)>(p.cells, sy, one);
+    if constexpr (sizeof(T) == 4)
+        return p.kv == 1 ? res_kernel_upto<T, 1, kResAcc / n>(p.cells, sy, one) : res_kernel_upto<T, 2, 1>(p.cells, sy, one);
+    if (p.kv == 1) return res_kernel_upto<T, 1, 2>(p.cells, sy, one);
+    return p.kv == 2 ? res_kernel_upto<T, 2, kResAcc / (2 * n)>(p.cells, sy, one) : res_kernel_upto<T, 4, 1>(p.cells, sy, one);
+}
+// cells of a pass at most, by columns per thread: 0 where there is no instance
+int res_cells(int elem_size, int kv) {
+    if (elem_size == 4) return kv == 1 ? 6 : (kv == 2 ? 1 : 0);
+    return kv == 1 ? 2 : (kv == 2 ? 6 : (kv == 4 ? 1 : 0));
 }
 
 }  // namespace
@@ -419,13 +430,13 @@ int resident_smem_bytes(const GainPass& p, int elem_size, int g_bytes, int f_len
 }
 
 // The pass over the resident units: gain_pass's columns per thread and the cells that the
-// accumulators allow, split evenly.
+// accumulators allow, split evenly (no cells: no such instance).
 GainPass resident_pass(int elem_size, const GainPass& g, int n_space) {
-    const int most = std::max(1, kResAcc / (g.kv * (16 / elem_size)));
-    const int passes = (n_space + most - 1) / most;
+    const int most = res_cells(elem_size, g.kv);
+    const int passes = most > 0 ? (n_space + most - 1) / most : 0;
     GainPass p;
     p.kv = g.kv;
-    p.cells = (n_space + passes - 1) / passes;
+    p.cells = passes > 0 ? (n_space + passes - 1) / passes : 0;
     return p;
 }
 

@@ -40,3 +40,27 @@ def test_large_contraction(cuda, prec, n2, n1):
                                                 ("f64", 4, 256, 8), ("f64", 8, 129, 8), ("f64", 7, 250, 8)])
 def test_cells_on_long_rows(cuda, prec, cells, p_g, u_g):
     _check(_cells_workload((2, 1, p_g, u_g), cells, 8, flux=False), prec, steps=2)
+
+
+@pytest.mark.parametrize("prec,cells,p_e,p_g", [("f32", 1, 4, 129), ("f32", 1, 2, 239), ("f32", 7, 4, 20), ("f64", 1, 3, 129),
+                                                ("f64", 1, 4, 70), ("f64", 1, 9, 79), ("f64", 2, 3, 66), ("f64", 2, 3, 60),
+                                                ("f64", 2, 3, 119), ("f64", 3, 5, 30), ("f64", 3, 2, 79), ("f64", 7, 6, 10)])
+def test_runs_on_long_rows_equal_steps(cuda, prec, cells, p_e, p_g):
+    """Runs of 66 steps with the gain in shared memory, every columns-per-thread variant and both state
+    lengths per thread, bit for bit against single steps."""
+    import numpy as np
+    from dtb.stepping import ForwardEulerStruct
+    w = _cells_workload((p_e, 1, p_g, 8), cells, 9, flux=False)
+    a, b = (ForwardEulerStruct(w.ps, w.f0, w.inj, w.binm, w.emim, w.fluxm,
+                               Precision=np.float64 if prec == "f64" else np.float32) for _ in range(2))
+    dt = np.random.default_rng(5).uniform(0.5, 1.0, 66)
+    n0, n1 = ctypes.c_int64(), ctypes.c_int64()
+    a.L.dtb_launch_count(a.ctx, ctypes.byref(n0))
+    a.run(dt)
+    a.L.dtb_launch_count(a.ctx, ctypes.byref(n1))
+    assert n1.value - n0.value == 4
+    for x in dt:
+        b(0.0, 1e9, float(x), 0)
+    np.testing.assert_array_equal(a.f, b.f)
+    a.close()
+    b.close()
