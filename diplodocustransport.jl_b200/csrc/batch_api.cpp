@@ -150,9 +150,11 @@ double ord_dec_host(unsigned long long e) {
 // ---------------------------------------------------------------- gain GEMM plans
 namespace {
 
-// Plans chosen so far in this process, by shape; a cache file (dtb_set_tune_cache) seeds it and
-// records what the autotuner measures, one line per shape:
-//   sm<SMs>:M<rows>:N1<n1>:n2<n2>:cols<columns>:cells<cells> <pair> <bn> <splits> <us>
+// Plans chosen so far in this process; a cache file (dtb_set_tune_cache) seeds them and records what
+// the autotuner measures, one line per shape and epilogue:
+//   sm<SMs>:M<rows>:N1<n1>:n2<n2>:cols<columns>:cells<cells> <pair> <bn> <splits> <us> <epilogue>
+// A plan is timed with the epilogue that gathers its partials, so it holds for that epilogue; a line
+// without the last field is for every epilogue. Keys: shape, or "shape epilogue".
 std::mutex g_plan_mu;
 std::map<std::string, GemmPlan> g_plans;
 std::string g_plan_file;
@@ -319,21 +321,22 @@ int tune_group(dtb_ctx* c, MixedGroup& G, const GemmShape& g, GemmPlan* best) {
     return rc;
 }
 
-// Plan of every gain group: a plan already chosen for the shape in this process (or read from
-// the cache file), else the autotuner's (or, with DTB_FLAG_NO_AUTOTUNE, the heuristic's).
-int plan_gemms(dtb_ctx* c, int Bcols, int max_pairs) {
+// Plan of every gain group: a plan already chosen for the shape and epilogue in this process (or
+// read from the cache file), else the autotuner's (or, with DTB_FLAG_NO_AUTOTUNE, the heuristic's).
+int plan_gemms(dtb_ctx* c, const std::string& epilogue, int Bcols, int max_pairs) {
     MixedState* m = c->mixed;
     const bool tune = (c->opts.flags & DTB_FLAG_NO_AUTOTUNE) == 0;
     for (auto& G : m->groups) {
         GemmPlan p;
         bool have = false;
         const GemmShape g = gemm_shape(c, G, Bcols, max_pairs);
-        const std::string key = plan_key(c, G, Bcols);
+        const std::string key = plan_key(c, G, Bcols), own = key + " " + epilogue;
         // held across lookup, tuning and store: concurrent commits of one shape get one plan
         std::unique_lock<std::mutex> lk(g_plan_mu, std::defer_lock);
         if (tune) {
             lk.lock();
-            auto it = g_plans.find(key);
+            auto it = g_plans.find(own);
+            if (it == g_plans.end()) it = g_plans.find(key);
             if (it != g_plans.end() && gemm_plan_valid(g, it->second)) {
                 p = it->second;
                 have = true;
@@ -342,10 +345,11 @@ int plan_gemms(dtb_ctx* c, int Bcols, int max_pairs) {
         if (!have) {
             if (tune) {
                 DTB_TRY(tune_group(c, G, g, &p));
-                g_plans[key] = p;
+                g_plans[own] = p;
                 if (!g_plan_file.empty()) {
                     if (FILE* f = std::fopen(g_plan_file.c_str(), "a")) {
-                        std::fprintf(f, "%s %d %d %d %.3f\n", key.c_str(), p.pair, p.bn, p.splits, p.us);
+                        std::fprintf(f, "%s %d %d %d %.3f %s\n", key.c_str(), p.pair, p.bn, p.splits, p.us,
+                                     epilogue.c_str());
                         std::fclose(f);
                     }
                 }
@@ -735,6 +739,7 @@ int commit_mixed(dtb_ctx* c) {
         ops.grp_sig1[gi] = m->sig + (size_t)G.in1 * B;
         ops.grp_sig2[gi] = m->sig + (size_t)G.in2 * B;
     }
+    std::string epilogue;
     // Row tiles: consecutive rows of one species and cell. Loss and emission run as tile products
     // where every row of the tile has the same list of emission pieces, so a tile also ends where
     // that list changes (not before its eighth row: shorter pieces keep the direct products).
@@ -842,6 +847,20 @@ int commit_mixed(dtb_ctx* c) {
             }
             tiles[(size_t)t].njobs = k;
         }
+        // what the epilogue's time depends on beside the groups: tiles, state, flux, loss and emission
+        // chunks
+        int n_jobs = 0, n_fast = 0;
+        for (int t = 0; t < n_tiles_r; ++t) {
+            n_fast += tiles[(size_t)t].fast;
+            for (int q = 0; q < tiles[(size_t)t].njobs; ++q) {
+                const RowJob& J = jobs[(size_t)t * kRowsMaxJobs + q];
+                n_jobs += (J.TL ? 1 : 0) + (J.TE ? 1 : 0);
+            }
+        }
+        char e[160];
+        std::snprintf(e, sizeof(e), "rows%dx%d:state%d:ell%d:jobs%d:fast%d", ops.tile_dim, n_tiles_r, n_st, ops.ell_w,
+                      n_jobs, n_fast);
+        epilogue = e;
         RowJob* d_jobs;
         RowTile* d_tiles;
         DTB_TRY(copy_host_ints(c, &d_jobs, jobs));
@@ -857,7 +876,7 @@ int commit_mixed(dtb_ctx* c) {
     ops.min_ratio = m->min_ratio;
     ops.nonfinite = m->nonfinite;
     // ---------------- GEMM plan per group: tile width, kernel and K splits (autotuned)
-    DTB_TRY(plan_gemms(c, Bcols, max_pairs));
+    DTB_TRY(plan_gemms(c, epilogue, Bcols, max_pairs));
     for (size_t gi = 0; gi < m->groups.size(); ++gi) set_group_ops(ops, m->groups[gi], (int)gi);
     for (auto& G : m->groups) c->gain_bytes += G.bytes;
     DTB_CUDA(cudaDeviceSynchronize());
@@ -1400,9 +1419,12 @@ int32_t dtb_set_tune_cache(const char* path) {
     g_plan_file = path ? path : "";
     if (!path) return DTB_OK;
     if (FILE* f = std::fopen(path, "r")) {
-        char key[160];
+        char line[512], key[160], epilogue[160];
         GemmPlan p;
-        while (std::fscanf(f, "%159s %d %d %d %lf", key, &p.pair, &p.bn, &p.splits, &p.us) == 5) g_plans[key] = p;
+        while (std::fgets(line, sizeof(line), f)) {
+            const int n = std::sscanf(line, "%159s %d %d %d %lf %159s", key, &p.pair, &p.bn, &p.splits, &p.us, epilogue);
+            if (n >= 5) g_plans[n == 6 ? std::string(key) + " " + epilogue : key] = p;
+        }
         std::fclose(f);
     }
     return DTB_OK;

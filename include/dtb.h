@@ -318,10 +318,13 @@ int32_t dtb_batch_gemm_stats(dtb_ctx* ctx, double* avg_ms, double* flops_per_ste
  * blocks of one input pair), the candidate plans on the device with CUDA events: the column
  * tile width (64, 128 or 256 instances), one SM per tile or an SM pair sharing 256 x 256 MMAs
  * (cta_group::2, when the group's 128-row tiles pair up) and the K splits that fill the device,
- * and keeps the fastest. A plan is chosen once per shape and process, so contexts of one shape
- * run the same plan (and round alike). dtb_set_tune_cache names a text file that seeds the
- * plans and records every measured one, one line per shape:
- *   sm<SMs>:M<rows>:N1<n1>:n2<n2>:cols<columns>:cells<cells> <pair 0|1> <bn> <splits> <us>
+ * and keeps the fastest with the epilogue that follows. A plan is chosen once per shape, epilogue
+ * (row tiles, flux width, loss and emission work) and process, so contexts of one grid run the same
+ * plan (and round alike). dtb_set_tune_cache names a text file that seeds the plans and records every
+ * measured one, one line per shape and epilogue:
+ *   sm<SMs>:M<rows>:N1<n1>:n2<n2>:cols<columns>:cells<cells> <pair 0|1> <bn> <splits> <us> <epilogue>
+ * A line without the last field holds for every epilogue. A plan whose accumulators would sum more
+ * than the autotuner's bound is measured afresh.
  * NULL forgets the plans chosen so far and stops recording. Process-wide; replaces the
  * per-stage tile choices of a hand-tuned build (no reference counterpart: the reference's
  * mul! calls, SteppingMethods.jl:372-373, leave this to MKL / cuBLAS). */

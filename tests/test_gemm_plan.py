@@ -111,3 +111,39 @@ def test_cached_plan_past_the_bound_is_measured_afresh(cuda, tmp_path):
             f, _, _ = ops.step(f, float(w.dt[i]), 0)
         assert np.max(np.abs(m.get_f(i) - f)) / np.max(np.abs(f)) <= 1e-5
     m.close()
+
+
+@pytest.mark.gpu
+def test_plans_belong_to_their_epilogue(cuda, tmp_path):
+    """Two grids with equal gain blocks and different epilogues (one without emission) are timed each for
+    itself: a cache line each, with its epilogue in the last field. A third context takes the plan of the
+    first's line, a line without that field serves both."""
+    B = 40
+    w = synth.batched_two_species(16, 1e-2, 1e2, 8, B, seed=32)
+    cache = tmp_path / "plans.txt"
+
+    def commit(emission):
+        from dtb.structs import EmissionMatrices
+        m = BatchedEuler(w.ps, w.inj, w.binm, w.emim if emission else EmissionMatrices(), w.fluxm, B)
+        p = m.gemm_plan(0)
+        m.close()
+        return p
+
+    set_tune_cache(str(cache))
+    try:
+        plans = [commit(True), commit(False), commit(True)]
+        lines = [ln.split() for ln in cache.read_text().splitlines()]
+        assert len(lines) == 2 and all(len(ln) == 6 for ln in lines)
+        assert lines[0][0] == lines[1][0] and lines[0][5] != lines[1][5]
+        assert plans[2] == plans[0]
+        # the recorded lines seed a new table; a line of the shape alone serves every epilogue
+        key = lines[0][0]
+        for text, plan in ((" ".join([key, "0", "64", "40", "7.0", lines[0][5]]), (False, 64, 40)),
+                           (f"{key} 0 64 36 7.0", (False, 64, 36))):
+            cache.write_text(text + "\n")
+            set_tune_cache(str(cache))
+            got = commit(True)
+            assert (got["pair"], got["bn"], got["n_splits"]) == plan
+        assert commit(False)["n_splits"] == 36
+    finally:
+        set_tune_cache(None)
