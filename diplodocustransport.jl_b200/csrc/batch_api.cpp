@@ -278,36 +278,37 @@ int tune_group(dtb_ctx* c, MixedGroup& G, const GemmShape& g, GemmPlan* best) {
     }
     const int all = g.cols;
     DTB_CUDA(cudaMemcpyAsync(m->active_hi, &all, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    double best_ms = 1e30;
-    int rc = DTB_OK;
-    for (const GemmPlan& p : cands) {
+    // a plan's GEMM and epilogue (rows), or its GEMM alone; ms per pass, negative when it cannot launch
+    const auto time_plan = [&](const GemmPlan& p, bool rows) {
         apply_plan(G, g, p);
         G.partial = part;
         set_group_ops(ops, G, gi);
         constexpr int kWarm = 2, kRep = 5;
-        float ms[2] = {0, 0};  // per GEMM, per GEMM and epilogue
+        float ms = 0;
         cudaError_t e = cudaSuccess;
-        for (int rows = 0; rows < 2 && e == cudaSuccess; ++rows) {
-            for (int k = 0; k < kWarm + kRep && e == cudaSuccess; ++k) {
-                if (k == kWarm) e = cudaEventRecord(e0, c->stream);
-                if (e == cudaSuccess) e = launch_group_gemm(c, G, m->F[0]);
-                if (e == cudaSuccess && rows)
-                    e = launch_mixed_rows(ops, m->F[0], m->C[0], m->F[1], m->C[1], m->gstep, 0, c->stream);
-            }
-            if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
-            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms[rows], e0, e1);
+        for (int k = 0; k < kWarm + kRep && e == cudaSuccess; ++k) {
+            if (k == kWarm) e = cudaEventRecord(e0, c->stream);
+            if (e == cudaSuccess) e = launch_group_gemm(c, G, m->F[0]);
+            if (e == cudaSuccess && rows)
+                e = launch_mixed_rows(ops, m->F[0], m->C[0], m->F[1], m->C[1], m->gstep, 0, c->stream);
         }
-        if (e != cudaSuccess) {  // a plan this device cannot launch is skipped
-            cudaGetLastError();
-            continue;
-        }
-        if (ms[1] / kRep < best_ms) {
-            best_ms = ms[1] / kRep;
+        if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+        if (e == cudaSuccess) return ms / kRep;
+        cudaGetLastError();
+        return -1.0f;
+    };
+    float best_ms = -1.0f;
+    int rc = DTB_OK;
+    for (const GemmPlan& p : cands) {
+        const float ms = time_plan(p, true);  // a plan this device cannot launch is skipped
+        if (ms >= 0 && (best_ms < 0 || ms < best_ms)) {
+            best_ms = ms;
             *best = p;
-            best->us = ms[0] / kRep * 1e3;
         }
     }
+    if (best_ms >= 0) best->us = std::max(0.0f, time_plan(*best, false)) * 1e3;
     const int zero = 0;
     cudaError_t e = cudaMemcpyAsync(m->active_hi, &zero, sizeof(int), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
