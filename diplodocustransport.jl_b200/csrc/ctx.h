@@ -167,6 +167,7 @@ struct dtb_ctx {
     int* sp_off_dev = nullptr;
     double* mom_w = nullptr;
     double* mom_out = nullptr;
+    double* mom_save = nullptr;  // kMomSaveBytes of a Solve's moments, from its first Solve with moments on
     int sp_off_host[2 * DTB_MAX_SPECIES + 2]{};
     RowOps<double> ops_d{};
     RowOps<float> ops_f{};
