@@ -59,3 +59,30 @@ def test_contexts_of_different_sizes_run_in_turn(cuda, prec, graph_steps, large,
             _contract(24, 8, prec)
     a.close()
     b.close()
+
+
+def test_contexts_run_at_once_on_their_own_threads(cuda):
+    """Three contexts on their own streams and host threads, two that keep the gain in shared memory (every
+    block of a launch waits for the others) and one that streams: each ends in the bits it has alone."""
+    import threading
+    cases = [((16, 8, 16, 8), "f64", 0), ((13, 8, 12, 8), "f32", 0), ((8, 8, 8, 8), "f64", 16)]
+    ms = [_method(*c) for c in cases]
+    dt = np.linspace(0.5, 1.0, 200)
+
+    def drive(m):
+        m.reset()
+        for _ in range(5):
+            m.run(dt)
+            m(0.0, 1e9, 0.75, 1)
+        return m.f
+
+    alone, at_once = [drive(m) for m in ms], [None] * len(ms)
+    threads = [threading.Thread(target=lambda k=k: at_once.__setitem__(k, drive(ms[k]))) for k in range(len(ms))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for x, y in zip(alone, at_once):
+        np.testing.assert_array_equal(x, y)
+    for m in ms:
+        m.close()
