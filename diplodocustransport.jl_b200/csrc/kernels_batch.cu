@@ -808,7 +808,7 @@ constexpr int kOP = kCK + 8;      // BF16 row pitch of a staged operand chunk (2
 constexpr int kRowStages = 3;     // cp.async ring depth
 constexpr int kEllFast = 8;       // ELL widths up to this take the hoisted-load flux path
 constexpr int kGatherVec = 18;    // 16-byte split partials in flight per thread in the gain gather
-constexpr int kGatherRow = 8;    // the same where a thread's four rows need a load each
+constexpr int kGatherRow = 4;     // splits in flight where its four rows need a load each (eight: no faster)
 
 // A tile of RT rows x IT instances on NW warps.
 template <int RT, int IT, int NW>
