@@ -22,13 +22,13 @@
 // The work table, the sums' order and the rows' arithmetic are those of gain_stream, euler_rows and
 // sympl_space, so states and step records agree bit for bit with steps run one by one.
 //
-// The launch is cooperative (the blocks wait on one another), every wait is bounded. Per step, against
-// the two launches: 2 x 128 FP64 states in intervals of 100 steps, 5.8 against 10.3 us; five FP32
-// cells of 140 + 126 states, symplectic, 12.4 against 15.4; two cells of a sparse 2 x 84-state FP64
-// grid, 6.5 against 8.3. A step of the first takes about 10,500 clocks: 4,700 for the units (shared
-// memory and a chain of latencies per unit, 16 warps), 2,500 for the sums and rows, the rest for
-// words on their way. Three groups of unit warps at 72 registers (spills), rows handed out
-// dynamically and one task per warp in the update were slower.
+// The launch is cooperative (the blocks wait on one another), every wait is bounded. Per step of long
+// runs, against the two launches: 2 x 128 FP64 states 5.1 against 9.2 us; five FP32 cells of 140 + 126
+// states, symplectic, 11.6 against 15.3; two cells of a sparse 2 x 84-state FP64 grid, 5.9 against 8.2.
+// A step of the first takes about 9,900 clocks: 4,700 for the units (shared memory and a chain of
+// latencies per unit, 16 warps), 2,500 for the sums and rows, the rest for words on their way. Three
+// groups of unit warps at 72 registers (spills), rows handed out dynamically and one task per warp in
+// the update were slower.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
