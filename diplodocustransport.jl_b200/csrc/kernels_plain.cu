@@ -95,11 +95,12 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
     if (warp == kGainConsumerWarps) {
         // ---------------- producer: one thread issues the bulk copies
         if (lane == 0) {
-            uint32_t it = 0, lk = 0;
+            uint32_t it = 0;
+            int slot = 0;  // the unit's place in the ring
             bool ok = true;
             GainUnit N{};
             if ((int)blockIdx.x < n_units) N = units[blockIdx.x];
-            for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++lk) {
+            for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, slot = slot + 1 == kRedRing ? 0 : slot + 1) {
                 const GainUnit U = N;
                 if (u + (int)gridDim.x < n_units) N = units[u + gridDim.x];  // in flight beside this unit
                 if (bad(U)) {
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
                     }
                     // the record reaches the consumers with the unit's first tile
                     if (t == 0)
-                        unit_s[lk % kRedRing] = {(unsigned short)U.b_off, (unsigned short)U.c_off, U.nb, U.n2p, U.tile_b};
+                        unit_s[slot] = {(unsigned short)U.b_off, (unsigned short)U.c_off, U.nb, U.n2p, U.tile_b};
                     const int rows = min(U.tile_b, U.nb - t * U.tile_b);
                     const uint32_t bytes = (uint32_t)rows * (uint32_t)U.n2p * (uint32_t)sizeof(T);
                     mbar_arrive_expect_tx(smem_u32(&full[st]), bytes);
@@ -147,11 +148,11 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
     stage_f<T, C>(f_s, f, so, f_len, n_mom, cell_list, cell0, n_cells, tid, kGainConsumers);
     asm volatile("bar.sync 1, %0;" ::"n"(kGainConsumers) : "memory");  // the consumer warps only
     uint32_t it = 0;
-    uint32_t lk = 0;  // units done by this block
+    int slot = 0;  // the unit's place in the ring, and the parity of its phase there
+    uint32_t unit_ph = 0;
     UnitSum<T, C, KV> sum;
     int c_off = -1, n2p = 0;  // the columns in sum's x
-    for (int u = blockIdx.x; u < n_units; u += gridDim.x, ++lk) {
-        const int slot = lk % kRedRing;
+    for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
         const GainRec* U = &unit_s[slot];  // valid from the unit's first tile on
         UnitMap m{};
         const S* f1 = f_s;
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&unit_bar[slot]));
         if (warp == 0) {
-            if (!mbar_wait_bounded(smem_u32(&unit_bar[slot]), (lk / kRedRing) & 1u, abort_flag)) {
+            if (!mbar_wait_bounded(smem_u32(&unit_bar[slot]), unit_ph, abort_flag)) {
                 if (!*abort_flag) atomicOr(err, KERR_TIMEOUT_FULL);
                 *abort_flag = 1;
                 return;
@@ -203,6 +204,10 @@ __global__ void __launch_bounds__(kGainThreads, 2) gain_stream_kernel(const T* _
                 const int cell = cell_list ? cell_list[cell0 + lane] : cell0 + lane;
                 partial[(size_t)cell * n_units + u] = s;
             }
+        }
+        if (++slot == kRedRing) {
+            slot = 0;
+            unit_ph ^= 1u;
         }
     }
 }
@@ -225,8 +230,10 @@ GainKernel<T> gain_kernel(const GainPass& p) {
     constexpr int n = Vec<T>::n;
     if (p.kv == 1) return gain_kernel_upto<T, 1, sizeof(T) == 8 ? 2 : 8>(p.cells);
     if (p.kv == 2) return gain_kernel_upto<T, 2, 32 / (2 * n)>(p.cells);
-    if constexpr (sizeof(T) == 8) return gain_kernel_upto<T, 4, 4>(p.cells);
-    return p.kv == 3 ? gain_stream_kernel<T, 1, 3> : gain_stream_kernel<T, 1, 4>;
+    if constexpr (sizeof(T) == 8)
+        return gain_kernel_upto<T, 4, 4>(p.cells);
+    else
+        return p.kv == 3 ? gain_stream_kernel<T, 1, 3> : gain_stream_kernel<T, 1, 4>;
 }
 
 template <typename T>

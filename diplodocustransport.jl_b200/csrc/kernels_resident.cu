@@ -409,10 +409,13 @@ template <typename T>
 ResKernel<T> res_kernel(const GainPass& p, bool sy, int n_state) {
     constexpr int n = Vec<T>::n;
     const bool one = n_state <= kResThreads;
-    if constexpr (sizeof(T) == 4)
+    if constexpr (sizeof(T) == 4) {
         return p.kv == 1 ? res_kernel_upto<T, 1, kResAcc / n>(p.cells, sy, one) : res_kernel_upto<T, 2, 1>(p.cells, sy, one);
-    if (p.kv == 1) return res_kernel_upto<T, 1, 2>(p.cells, sy, one);
-    return p.kv == 2 ? res_kernel_upto<T, 2, kResAcc / (2 * n)>(p.cells, sy, one) : res_kernel_upto<T, 4, 1>(p.cells, sy, one);
+    } else {
+        if (p.kv == 1) return res_kernel_upto<T, 1, 2>(p.cells, sy, one);
+        return p.kv == 2 ? res_kernel_upto<T, 2, kResAcc / (2 * n)>(p.cells, sy, one)
+                         : res_kernel_upto<T, 4, 1>(p.cells, sy, one);
+    }
 }
 // cells of a pass at most, by columns per thread: 0 where there is no instance
 int res_cells(int elem_size, int kv) {
